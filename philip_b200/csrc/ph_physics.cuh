@@ -71,10 +71,13 @@ template <typename R> __device__ __forceinline__ R rabs(R x) { return x < R(0) ?
 
 // Quotient used inside the flux functions. PH_FAST_DIV=0: IEEE division. Otherwise the
 // numerator times the hardware approximate reciprocal (PTX rcp.approx.ftz.f64/.f32,
-// relative error about 1e-6 in FP64) refined by Newton-Raphson steps
-// r <- r + r (1 - b r), each of which squares the relative error: two steps in FP64
-// (about 2 ulp, measured against IEEE division in tests/test_gpu_quotient.py), none
-// in FP32 (the f32 approximation is within about 1 ulp already).
+// relative error about 1e-6 in FP64), refined in FP64 by one step of the third-order iteration
+// r <- r (1 + e + e^2), e = 1 - b r (the hyperpower method: the error becomes e^3, about 1e-18),
+// measured against IEEE division in tests/test_gpu_quotient.py (about 2 ulp); not refined in FP32
+// (the f32 approximation is within about 1 ulp already). Three dependent operations instead of
+// the four of two Newton-Raphson steps: the divisions sit on the critical path of every pair flux
+// (node-per-lane stage kernel at 24^3 cells, p = 5: 0.488 ms against 0.497, 32^3, p = 3: 0.385
+// against 0.393; GL flux nodes 24^3, p = 5: a step 11.79 against 11.89 ms).
 #ifndef PH_FAST_DIV
 #define PH_FAST_DIV 1
 #endif
@@ -93,10 +96,9 @@ template <> __device__ __forceinline__ double qrcp<double>(double b) {
 #if PH_FAST_DIV == 0
     return 1.0 / b;
 #else
-    double r = rcp_approx(b);
-    r = fma(r, fma(-b, r, 1.0), r);
-    r = fma(r, fma(-b, r, 1.0), r);
-    return r;
+    const double r = rcp_approx(b);
+    const double e = fma(-b, r, 1.0);
+    return fma(r, fma(e, e, e), r);
 #endif
 }
 template <> __device__ __forceinline__ float qrcp<float>(float b) {
