@@ -29,6 +29,27 @@ static cudaError_t launch_one(const StageArgs& a, cudaStream_t s) {
     return cudaGetLastError();
 }
 
+template <typename R, int N1, bool VISC, bool CURV>
+static cudaError_t launch_line(const StageArgs& a, cudaStream_t s) {
+    constexpr int CPC = line_cells<N1>();
+    using L = LineLayout<R, N1, CPC, CURV>;
+    constexpr size_t bytes = L::bytes;
+    auto kern = line_kernel<R, N1, CPC, VISC, CURV>;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    static bool configured[64] = {false};
+    if (dev < 64 && !configured[dev]) {
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+        if (e != cudaSuccess) return e;
+        configured[dev] = true;
+    }
+    const int cells = a.tiles ? a.ntiles * cells_per_cta<N1>() : a.nc - a.cell_begin;
+    const int grid = (cells + CPC - 1) / CPC;
+    if (grid <= 0) return a.tiles ? cudaSuccess : cudaErrorInvalidValue;
+    kern<<<grid, L::NT, bytes, s>>>(a, cells_per_cta<N1>());
+    return cudaGetLastError();
+}
+
 template <typename R, int N1>
 static cudaError_t launch_prec(const StageArgs& a, bool visc, bool split, cudaStream_t s) {
     // the Chandrashekar + EC/Roe (+ BR2) combination has its own compile-time instance; the
@@ -50,6 +71,10 @@ static cudaError_t launch_prec(const StageArgs& a, bool visc, bool split, cudaSt
         if (split) return hot ? launch_one<R, N1, false, true, 1, false, true>(a, s)
                               : launch_one<R, N1, false, true, 0, false, true>(a, s);
         return launch_one<R, N1, false, false, 0, false, true>(a, s);
+    }
+    if (hot && a.mode != 3) {   // (mode 3, the low-storage stages, has per-tile error sums of residual_kernel's tiles)
+        if (a.metric) return visc ? launch_line<R, N1, true, true>(a, s) : launch_line<R, N1, false, true>(a, s);
+        return visc ? launch_line<R, N1, true, false>(a, s) : launch_line<R, N1, false, false>(a, s);
     }
     if (a.metric) {   // curvilinear cells
         if (!split) return visc ? launch_one<R, N1, true, false, 0, true>(a, s) : launch_one<R, N1, false, false, 0, true>(a, s);
@@ -75,12 +100,25 @@ template <int N1, int V> constexpr int batched_cpc() {
     return N1 == 2 ? 16 : N1 == 3 ? (V == 0 ? 4 : 8) : N1 == 4 ? (V == 0 ? 2 : 4) : N1 == 5 ? (V == 0 ? 1 : 2) : 1;
 }
 
+// the batched kernel of a group: the line form for the Chandrashekar + EC/Roe flux set without boundary
+// faces, else the node-per-lane form
+template <typename R, int N1, int V, int FS, bool CURV, bool BND> struct BatchedKernel {
+    static constexpr int CPC = batched_cpc<N1, V>();
+    using L = Layout<R, N1, CPC, false, true, CURV>;
+    static auto get() { return residual_kernel_batched<R, N1, CPC, false, true, FS, CURV, BND>; }
+};
+template <typename R, int N1, int V, bool CURV> struct BatchedKernel<R, N1, V, 1, CURV, false> {
+    static constexpr int CPC = batched_cpc<N1, V>();
+    using L = LineLayout<R, N1, CPC, CURV>;
+    static auto get() { return line_kernel_batched<R, N1, CPC, CURV>; }
+};
+
 template <typename R, int N1, int V, int FS, bool CURV, bool BND>
 static cudaError_t launch_batched_one(const StageArgs* inst, const BatchTile* tiles, int ntiles, int grid,
                                       cudaStream_t s) {
-    constexpr int CPC = batched_cpc<N1, V>();
-    using L = Layout<R, N1, CPC, false, true, CURV>;
-    auto kern = residual_kernel_batched<R, N1, CPC, false, true, FS, CURV, BND>;
+    using K = BatchedKernel<R, N1, V, FS, CURV, BND>;
+    using L = typename K::L;
+    auto kern = K::get();
     int dev = 0;
     cudaGetDevice(&dev);
     static bool configured[64] = {false};
@@ -138,10 +176,10 @@ cudaError_t launch_stage_batched(const StageArgs* inst, const BatchTile* tiles, 
 
 template <typename R, int N1, int V, bool CURV>
 static bool batched_shape_one(int* cpc, int* threads, size_t* smem, int* ctas_per_sm) {
-    constexpr int CPC = batched_cpc<N1, V>();
-    using L = Layout<R, N1, CPC, false, true, CURV>;
-    *cpc = CPC; *threads = L::NT; *smem = L::bytes;
-    auto kern = residual_kernel_batched<R, N1, CPC, false, true, 1, CURV>;
+    using K = BatchedKernel<R, N1, V, 1, CURV, false>;
+    using L = typename K::L;
+    *cpc = K::CPC; *threads = L::NT; *smem = L::bytes;
+    auto kern = K::get();
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::bytes) != cudaSuccess) return false;
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(ctas_per_sm, kern, L::NT, L::bytes) == cudaSuccess;
 }

@@ -298,7 +298,7 @@ __device__ __forceinline__ void face_item(const Cst<R>& cst, int tp, int cf, int
         const R nrm[3] = {qdiv<R>(m[0], J), qdiv<R>(m[1], J), qdiv<R>(m[2], J)};
         NodeQ<R> qo, qe;
         load_q<R>(sD + c * NQS * NP, NP, node, qo);
-        node_prepare<R>(ue, tp, cst.gm1, qe, nullptr);
+        node_prepare<R, LOG_STORED, N1 % 2 == 0>(ue, tp, cst.gm1, qe, nullptr);
         R F[5];
         if (plus) conv_num_flux_n<R>(uo, ue, qo, qe, nrm, tp, cf, cst, F);
         else conv_num_flux_n<R>(ue, uo, qe, qo, nrm, tp, cf, cst, F);
@@ -329,7 +329,7 @@ __device__ __forceinline__ void face_item(const Cst<R>& cst, int tp, int cf, int
     rotate_state<R>(ue, d, re);
     NodeQ<R> qo, qe;
     load_q_rot<R>(sD + c * NQS * NP, NP, node, d, qo);
-    node_prepare<R>(re, tp, cst.gm1, qe, nullptr);
+    node_prepare<R, LOG_STORED, N1 % 2 == 0>(re, tp, cst.gm1, qe, nullptr);
     R Fr[5], Fs[5];
     if (plus) conv_num_flux<R, 0>(ro, re, qo, qe, tp, cf, cst, Fr);
     else conv_num_flux<R, 0>(re, ro, qe, qo, tp, cf, cst, Fr);

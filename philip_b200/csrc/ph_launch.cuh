@@ -3,6 +3,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include "ph_kernels.cuh"
+#include "ph_lines.cuh"
 #include "ph_gl.cuh"
 #include "ph_limiter.cuh"
 #include "ph_integrals.cuh"

@@ -143,6 +143,12 @@ template <typename R> __device__ __forceinline__ R pressure_ieee(const R u[5], R
     return positive<R>(gm1 * (u[4] - R(0.5) * rho * v2), st);
 }
 
+// Where the logarithms of a logarithmic mean come from (the Chandrashekar flux): LOG_STORED, the
+// node quantities la / lb; LOG_HERE, taken where the series branch does not hold (smooth flow never
+// takes it, so nothing is spent on them); LOG_NONE, the caller has checked that every pair takes
+// the series. The three give the same bits.
+enum LogMode { LOG_STORED = 0, LOG_HERE = 1, LOG_NONE = 2 };
+
 // Per-node quantities reused by every two-point flux that touches the node.
 template <typename R> struct NodeQ {
     R rho, v[3], p, E;
@@ -150,17 +156,34 @@ template <typename R> struct NodeQ {
     R vsq;            // |v|^2 (CH, Ra) or specific total energy (KG)
 };
 
-template <typename R>
+// |v|^2 in the order v0^2 + v1^2 + v2^2. In FP32 the roundings are spelled out: left to the compiler,
+// v0^2 + v1^2 is fused in some kernels and not in others, and a solve's bits would depend on which
+// kernel works on its cells. FUSED: v1^2 fused onto v0^2 (v2^2 is fused in both).
+template <typename R, bool FUSED> __device__ __forceinline__ R sum_squares(const R v[3]) {
+    if constexpr (sizeof(R) == 4) {
+        const float a = __fmul_rn(v[0], v[0]);
+        return __fmaf_rn(v[2], v[2], FUSED ? __fmaf_rn(v[1], v[1], a) : __fadd_rn(a, __fmul_rn(v[1], v[1])));
+    } else {
+        R v2 = R(0);
+#pragma unroll
+        for (int d = 0; d < 3; ++d) v2 = v2 + v[d] * v[d];
+        return v2;
+    }
+}
+
+// FUSED: the rounding of |v|^2 in the precision form (a cell's own nodes: false; a face's neighbour
+// value: at even N1)
+template <typename R, int LM = LOG_STORED, bool FUSED = false>
 __device__ __forceinline__ void node_prepare(const R u[5], int tp, R gm1, NodeQ<R>& q, unsigned* st) {
     q.rho = u[0];
-    R v2 = R(0);
 #pragma unroll
-    for (int d = 0; d < 3; ++d) { q.v[d] = qdiv<R>(u[1 + d], u[0]); v2 = v2 + q.v[d] * q.v[d]; }
+    for (int d = 0; d < 3; ++d) q.v[d] = qdiv<R>(u[1 + d], u[0]);
+    const R v2 = sum_squares<R, FUSED>(q.v);
     q.E = u[4];
     q.p = positive<R>(gm1 * (u[4] - R(0.5) * u[0] * v2), st);
     if (tp == TP_CH) {
         q.a = q.rho; q.b = qdiv<R>(q.rho, R(2) * q.p);
-        q.la = rlog<R>(q.a); q.lb = rlog<R>(q.b);
+        if (LM == LOG_STORED) { q.la = rlog<R>(q.a); q.lb = rlog<R>(q.b); }
         q.vsq = q.v[0] * q.v[0] + q.v[1] * q.v[1] + q.v[2] * q.v[2];
     } else if (tp == TP_RA) {
         q.a = q.rho; q.b = qdiv<R>(q.rho, q.p);
@@ -208,7 +231,7 @@ template <typename R> __device__ __forceinline__ R log_mean_series(R u) {
 // Both logarithmic means follow log_mean (the same branch test, series for u < 1e-2), with
 // the quotients rearranged to share reciprocals: three when both means take the series
 // branch (smooth flow), at most five, where the plain form divides six times.
-template <typename R>
+template <typename R, int LM = LOG_STORED>
 __device__ __forceinline__ void ch_means(const NodeQ<R>& i, const NodeQ<R>& j, const Cst<R>& c, R& rho_log,
                                          R& p_hat, R& h0) {
     const R srho = i.rho + j.rho, drho = i.rho - j.rho;
@@ -218,19 +241,20 @@ __device__ __forceinline__ void ch_means(const NodeQ<R>& i, const NodeQ<R>& j, c
     R inv_blog;
     {
         const R f = db * rsb, u = f * f;
-        if (u < R(1.0e-2)) inv_blog = R(2) * log_mean_series<R>(u) * rsb;
+        if (LM == LOG_NONE || u < R(1.0e-2)) inv_blog = R(2) * log_mean_series<R>(u) * rsb;
+        else if (LM == LOG_HERE) inv_blog = (rlog<R>(i.b) - rlog<R>(j.b)) * qrcp<R>(db);
         else inv_blog = (i.lb - j.lb) * qrcp<R>(db);
     }
     R inv_rlog;
     {
         const R rs = qrcp<R>(srho);
         const R f = drho * rs, u = f * f;
-        if (u < R(1.0e-2)) {
+        if (LM == LOG_NONE || u < R(1.0e-2)) {
             const R F = log_mean_series<R>(u);
             inv_rlog = R(2) * F * rs;
             rho_log = R(0.5) * srho * qrcp<R>(F);
         } else {
-            const R dl = i.la - j.la;
+            const R dl = LM == LOG_HERE ? rlog<R>(i.rho) - rlog<R>(j.rho) : i.la - j.la;
             rho_log = drho * qrcp<R>(dl);
             inv_rlog = dl * qrcp<R>(drho);
         }
@@ -239,12 +263,12 @@ __device__ __forceinline__ void ch_means(const NodeQ<R>& i, const NodeQ<R>& j, c
 }
 
 // Two-point flux component along direction d (compile time) for all 5 equations.
-template <typename R, int d>
+template <typename R, int d, int LM = LOG_STORED>
 __device__ __forceinline__ void two_point_dir(const NodeQ<R>& i, const NodeQ<R>& j, int tp,
                                               const Cst<R>& c, R F[5]) {
     if (tp == TP_CH) {
         R rho_log, p_hat, h0;
-        ch_means<R>(i, j, c, rho_log, p_hat, h0);
+        ch_means<R, LM>(i, j, c, rho_log, p_hat, h0);
         R va[3], vsq = R(0);
 #pragma unroll
         for (int k = 0; k < 3; ++k) { va[k] = R(0.5) * (i.v[k] + j.v[k]); vsq += va[k] * va[k]; }
@@ -306,6 +330,74 @@ __device__ __forceinline__ void two_point_dir(const NodeQ<R>& i, const NodeQ<R>&
         F[1 + d] += p - c.shift();
         F[4] = m * e + p * v[d];
     }
+}
+
+// The Chandrashekar pair flux from halved node quantities, for kernels that evaluate many pairs per
+// node: with rho / 2, v / 2 and |v|^2 / 4 stored, the means' factors 1/2 and 1/4 and the doubled
+// series cost nothing (6 of about 63 operations per pair). Scaling by powers of two is exact, so the
+// flux has the bits of two_point_dir<R, 0> / two_point_n.
+template <typename R> struct HalfQ {
+    R hr, hv[3], b, q4;   // rho / 2, v / 2, rho / (2 p), |v|^2 / 4
+    R la, lb;             // logarithms of rho and b (LOG_STORED)
+};
+
+template <typename R, int LM>
+__device__ __forceinline__ void ch_means_half(const HalfQ<R>& i, const HalfQ<R>& j, const Cst<R>& c, R& rho_log,
+                                              R& p_hat, R& h0) {
+    const R hs = i.hr + j.hr, dh = i.hr - j.hr;
+    const R sb = i.b + j.b, db = i.b - j.b;
+    const R rsb = qrcp<R>(sb);
+    p_hat = hs * rsb;
+    R inv_hblog;   // half of ch_means' inv_blog
+    {
+        const R f = db * rsb, u = f * f;
+        if (LM == LOG_NONE || u < R(1.0e-2)) inv_hblog = log_mean_series<R>(u) * rsb;
+        else inv_hblog = R(0.5) * ((i.lb - j.lb) * qrcp<R>(db));
+    }
+    R inv_rlog;
+    {
+        const R rhs = qrcp<R>(hs);
+        const R f = dh * rhs, u = f * f;
+        if (LM == LOG_NONE || u < R(1.0e-2)) {
+            const R F = log_mean_series<R>(u);
+            inv_rlog = F * rhs;
+            rho_log = hs * qrcp<R>(F);
+        } else {
+            const R dl = i.la - j.la, drho = R(2) * dh;
+            rho_log = drho * qrcp<R>(dl);
+            inv_rlog = dl * qrcp<R>(drho);
+        }
+    }
+    h0 = inv_hblog * (R(2) * c.inv2gm1) + p_hat * inv_rlog - (i.q4 + j.q4);
+}
+// along the first axis of the frame the velocities are given in
+template <typename R, int LM>
+__device__ __forceinline__ void ch_pair_axis(const HalfQ<R>& i, const HalfQ<R>& j, const Cst<R>& c, R F[5]) {
+    R rho_log, p_hat, h0;
+    ch_means_half<R, LM>(i, j, c, rho_log, p_hat, h0);
+    R va[3], vsq = R(0);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) { va[k] = i.hv[k] + j.hv[k]; vsq += va[k] * va[k]; }
+    const R m = rho_log * va[0];
+    F[0] = m;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) F[1 + k] = m * va[k];
+    F[1] += p_hat - c.shift();
+    F[4] = m * (h0 + vsq);
+}
+// dotted with n
+template <typename R, int LM>
+__device__ __forceinline__ void ch_pair_n(const HalfQ<R>& i, const HalfQ<R>& j, const R n[3], const Cst<R>& c, R F[5]) {
+    R rho_log, p_hat, h0;
+    ch_means_half<R, LM>(i, j, c, rho_log, p_hat, h0);
+    R va[3], vsq = R(0), vn = R(0);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) { va[k] = i.hv[k] + j.hv[k]; vsq += va[k] * va[k]; vn += va[k] * n[k]; }
+    const R m = rho_log * vn;
+    F[0] = m;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) F[1 + k] = m * va[k] + (p_hat - c.shift()) * n[k];
+    F[4] = m * (h0 + vsq);
 }
 
 // Physical convective flux along direction d (p0: the precision form's pressure shift).
@@ -378,11 +470,11 @@ __device__ __forceinline__ void roe_dissipation(const NodeQ<R>& L, const NodeQ<R
 
 // Convective numerical flux dot n for n = +e_d, evaluated with L = minus side.
 // (convective_numerical_flux.cpp:35-54 composition of baseline + dissipation)
-template <typename R, int d>
+template <typename R, int d, int LM = LOG_STORED>
 __device__ __forceinline__ void conv_num_flux(const R uL[5], const R uR[5], const NodeQ<R>& L, const NodeQ<R>& Rq,
                                               int tp, int cf, const Cst<R>& c, R out[5]) {
     if (cf == CF_EC || cf == CF_EC_LXF || cf == CF_EC_ROE) {
-        two_point_dir<R, d>(L, Rq, tp, c, out);
+        two_point_dir<R, d, LM>(L, Rq, tp, c, out);
     } else {
         R FL[5], FR[5];
         conv_flux_dir<R, d>(L, c.shift(), FL);
@@ -409,12 +501,12 @@ __device__ __forceinline__ void conv_num_flux(const R uL[5], const R uR[5], cons
 // unit physical normal on faces (strong_dg.cpp:1235-1515, :3354-3452).
 
 // Two-point flux dotted with n.
-template <typename R>
+template <typename R, int LM = LOG_STORED>
 __device__ __forceinline__ void two_point_n(const NodeQ<R>& i, const NodeQ<R>& j, const R n[3], int tp,
                                             const Cst<R>& c, R F[5]) {
     if (tp == TP_CH) {
         R rho_log, p_hat, h0;
-        ch_means<R>(i, j, c, rho_log, p_hat, h0);
+        ch_means<R, LM>(i, j, c, rho_log, p_hat, h0);
         R va[3], vsq = R(0), vn = R(0);
 #pragma unroll
         for (int k = 0; k < 3; ++k) { va[k] = R(0.5) * (i.v[k] + j.v[k]); vsq += va[k] * va[k]; vn += va[k] * n[k]; }
@@ -542,11 +634,11 @@ __device__ __forceinline__ void roe_dissipation_n(const NodeQ<R>& L, const NodeQ
 }
 
 // Convective numerical flux dotted with the unit normal n (L = the side n points away from).
-template <typename R>
+template <typename R, int LM = LOG_STORED>
 __device__ __forceinline__ void conv_num_flux_n(const R uL[5], const R uR[5], const NodeQ<R>& L, const NodeQ<R>& Rq,
                                                 const R n[3], int tp, int cf, const Cst<R>& c, R out[5]) {
     if (cf == CF_EC || cf == CF_EC_LXF || cf == CF_EC_ROE) {
-        two_point_n<R>(L, Rq, n, tp, c, out);
+        two_point_n<R, LM>(L, Rq, n, tp, c, out);
     } else {
         R FL[5], FR[5];
         conv_flux_n<R>(L, n, c.shift(), FL);
