@@ -603,7 +603,19 @@ int build_gl_operators(const ph_params* prm, ph::GlTab& t, ph::OpTab& ops) {
     if (!mat_inv(MK, nd, MKi)) return fail(PH_ERR_INVALID, "singular FR mass matrix");
     if (kaux == 0.0) MKai = Mi;
     else if (!mat_inv(MKa, nd, MKai)) return fail(PH_ERR_INVALID, "singular auxiliary FR mass matrix");
-    for (int i = 0; i < nd * nd; ++i) { t.minv[i] = MKi[i]; t.minv_aux[i] = MKai[i]; }
+    // (M + K)^-1 folded into the transposed lifts: chi (M + K)^-1 and (M + K)^-1 chis (M + K is symmetric)
+    for (int i = 0; i < nd; ++i) {
+        for (int q = 0; q < nq; ++q) {
+            double v = 0.0;
+            for (int j = 0; j < nd; ++j) v += chi[q * nd + j] * MKi[j * nd + i];
+            t.chm[q * nd + i] = v;
+        }
+        for (int side = 0; side < 2; ++side) {
+            double v = 0.0;
+            for (int j = 0; j < nd; ++j) v += MKi[i * nd + j] * t.chis[side][j];
+            t.chms[side][i] = v;
+        }
+    }
     // chi (M + K_aux)^-1 chi^T (nq x nq): the auxiliary equation's inverse mass seen from the flux
     // nodes (solution values at the flux nodes of (M + K_aux)^-1 chi^T applied to flux-node data)
     for (int a = 0; a < nq; ++a)
@@ -1023,6 +1035,7 @@ struct ph_ctx {
     double* d_t1 = nullptr;
     double* d_t2 = nullptr;
     double* d_vis = nullptr;
+    double* d_proj = nullptr;
     double* d_glvm = nullptr;           // curvilinear uncollocated: [nc][10][nq^3] cofactor + 1 / det J
     double* d_glfn = nullptr;           // curvilinear uncollocated: [nc][6][3][nq^2] face metric columns
     // optional per-kernel timing: 1 = CUDA events around every direct launch, the stream
@@ -1247,7 +1260,7 @@ int dispatch_gl(ph_ctx* c, int kernel, const ph::StageArgs& a) {
     static const char* const kName[] = {"face-value kernel", "auxiliary kernel", "stage kernel",
                                         "inverse-mass kernel"};
     NvtxRange nvtx(kName[kernel]);
-    const ph::GlArgs g{c->d_gl, c->d_t1, c->d_t2, c->d_vis, c->d_glvm, c->d_glfn, c->d_fb};
+    const ph::GlArgs g{c->d_gl, c->d_t1, c->d_t2, c->d_vis, c->d_glvm, c->d_glfn, c->d_fb, c->d_proj};
     cudaError_t e;
     timer_begin(c);
     switch (c->N1) {
@@ -1650,8 +1663,9 @@ static int create_context(const ph_mesh_desc* mesh, const ph_params* prm, void* 
         bad |= dalloc(&c->d_t1, faces * (c->split ? 10 : 5));
         if (c->visc) {
             bad |= dalloc(&c->d_t2, faces * ph::GL_T2W);
-            bad |= dalloc(&c->d_vis, (size_t)c->nc * 4 * c->NP);
+            bad |= dalloc(&c->d_vis, (size_t)c->nc * 4 * c->NQ * c->NQ * c->NQ);
         }
+        if (c->split) bad |= dalloc(&c->d_proj, (size_t)c->nc * 5 * c->NQ * c->NQ * c->NQ);
         if (c->curv) {
             const size_t q3 = (size_t)c->NQ * c->NQ * c->NQ;
             bad |= dalloc(&c->d_glvm, (size_t)c->nc * 10 * q3);
@@ -1805,7 +1819,7 @@ int ph_ctx_destroy(ph_ctx* c) {
     void* ptrs[] = {c->d_nbr, c->d_ops, c->d_itab, c->d_sol, c->d_stA, c->d_stB, c->d_acc, c->d_carry,
                     c->d_fv, c->d_comp, c->d_tmpA, c->d_tmpB, c->d_partial, c->d_status, c->d_metric, c->d_xnode, c->d_origin, c->d_err,
                     c->d_table, c->d_counter, c->d_ent, c->d_ent_cell, c->d_halo, c->d_gl, c->d_t1, c->d_t2,
-                    c->d_vis, c->d_ltab, c->d_glvm, c->d_glfn, c->d_btype, c->d_fb, c->d_tiles};
+                    c->d_vis, c->d_proj, c->d_ltab, c->d_glvm, c->d_glfn, c->d_btype, c->d_fb, c->d_tiles};
     if (c->side) cudaStreamSynchronize(c->side);
     for (void* p : ptrs) if (p) cudaFree(p);
     if (c->side) cudaStreamDestroy(c->side);

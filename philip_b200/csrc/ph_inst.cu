@@ -369,7 +369,7 @@ static cudaError_t launch_gl_nq(int kernel, const StageArgs& a, const GlArgs& g,
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
     constexpr int NT = gl_threads<NQ>();
-    static bool cfg[27][64] = {};
+    static bool cfg[29][64] = {};
     if (kernel == 0) {
         if (split) return launch_gl_kernel(gl_trace_kernel<ND, NQ, true>, GlTraceLayout<ND, NQ, true>::bytes, NT, a, g, ht,
                                            cfg[0][dev], s);
@@ -440,6 +440,14 @@ static cudaError_t launch_gl_nq(int kernel, const StageArgs& a, const GlArgs& g,
         return launch_gl_kernel(gl_stage_kernel<ND, NQ, false, false, false, true>,
                                 GlStageLayout<ND, NQ, false, false>::bytes, NT, a, g, ht, cfg[20][dev], s);
     }
+    // the Chandrashekar + EC/Roe (+ BR2) flux set on line segments; the relaxation RK's entropy estimate
+    // lives in the general kernel
+    if (split && a.pc.two_point == TP_CH && a.pc.conv_flux == CF_EC_ROE && (!visc || a.pc.diss_flux == DF_BR2) &&
+        !a.ent_partial)
+        return visc ? launch_gl_kernel(gl_line_stage_kernel<ND, NQ, true>, GlLineLayout<ND, NQ>::bytes,
+                                       GlLineLayout<ND, NQ>::NT, a, g, ht, cfg[27][dev], s)
+                    : launch_gl_kernel(gl_line_stage_kernel<ND, NQ, false>, GlLineLayout<ND, NQ>::bytes,
+                                       GlLineLayout<ND, NQ>::NT, a, g, ht, cfg[28][dev], s);
     if (visc) {
         if (split) return launch_gl_kernel(gl_stage_kernel<ND, NQ, true, true>, GlStageLayout<ND, NQ, true, true>::bytes,
                                            NT, a, g, ht, cfg[4][dev], s);

@@ -32,12 +32,15 @@ template <int N1> constexpr int line_cells() {
     return N1 == 2 ? 16 : N1 == 3 ? 4 : N1 == 4 ? 4 : 1;
 }
 
+// nodes per lane, lanes per line, lines per warp (lane = place on the line * SPW + line of the warp)
+template <int N1> __host__ __device__ constexpr int line_npl() { return N1 % 2 == 0 ? 2 : 1; }
+template <int N1> __host__ __device__ constexpr int line_lanes() { return N1 / line_npl<N1>(); }
+template <int N1> __host__ __device__ constexpr int line_spw() { return 32 / line_lanes<N1>(); }
+
 template <typename R, int N1, int CPC, bool CURV>
 struct LineLayout {
     static constexpr int NP = N1 * N1 * N1, NF = N1 * N1;
-    static constexpr int NPL = N1 % 2 == 0 ? 2 : 1;           // nodes per lane
-    static constexpr int H = N1 / NPL;                        // lanes per line
-    static constexpr int SPW = 32 / H;                        // lines per warp
+    static constexpr int NPL = line_npl<N1>(), H = line_lanes<N1>(), SPW = line_spw<N1>();
     static constexpr int NT = (CPC * NF + SPW - 1) / SPW * 32;
     static constexpr int NQ = 8 + (CURV ? 9 : 0);   // rho/2 v/2 (3) p E b |v|^2/4 (+ half the metric cofactor)
     static constexpr bool F32 = sizeof(R) == 4;
@@ -77,11 +80,151 @@ template <typename R> __device__ __forceinline__ bool series_span(int lo, int hi
     return lo > 0 && (unsigned)hi - (unsigned)lo < lim;
 }
 
-// halved node quantities of node `o` (an offset into the rows) in a frame whose velocity rows are r1..r3
-template <typename R, int NS>
-__device__ __forceinline__ void line_q(const R* Q, int o, int r1, int r2, int r3, HalfQ<R>& q) {
-    q.hr = Q[o]; q.hv[0] = Q[r1 + o]; q.hv[1] = Q[r2 + o]; q.hv[2] = Q[r3 + o];
-    q.b = Q[6 * NS + o]; q.q4 = Q[7 * NS + o];
+// Where a cell's halved node quantities are: rho / 2 and the velocity rows at q (+ r1..r3: the rows of
+// the line's frame), b and |v|^2 / 4 from qb, the logarithms from l, the halved metric column from m.
+template <typename R> struct LineRows {
+    const R* q;
+    const R* qb;
+    const R* l;
+    const R* m;   // rows 0, 3, 6 of it (curvilinear cells)
+    int r1, r2, r3;
+};
+
+// The two-point terms of one line on its segment of lanes: acc[e][s] = sum_j S[i][j] F(i, j) for this lane's
+// nodes i = NPL pos + e, momentum in the line's frame (curvilinear: in x, y, z). Node i is at offset
+// base + i st of the rows (row pitch NS); sS the operator, row-major; pos, seg: the lane's place on the
+// line and its line of the warp. All lanes of the warp call it.
+template <typename R, int N1, int NS, bool CURV, int LM>
+__device__ __forceinline__ void line_pairs(const LineRows<R>& rw, int base, int st, int pos, int seg, const R* sS,
+                                           const Cst<R>& cst, R (&acc)[line_npl<N1>()][5]) {
+    constexpr int NPL = line_npl<N1>(), H = line_lanes<N1>(), SPW = line_spw<N1>();
+    const int prev = (pos == 0 ? H - 1 : pos - 1) * SPW + seg;
+    auto node = [&](int i, HalfQ<R>& q, R m[3]) {
+        const int o = base + i * st;
+        q.hr = rw.q[o]; q.hv[0] = rw.q[rw.r1 + o]; q.hv[1] = rw.q[rw.r2 + o]; q.hv[2] = rw.q[rw.r3 + o];
+        q.b = rw.qb[o]; q.q4 = rw.qb[NS + o];
+        if constexpr (LM == LOG_STORED) { q.la = rw.l[o]; q.lb = rw.l[NS + o]; }
+        if constexpr (CURV) {
+#pragma unroll
+            for (int k = 0; k < 3; ++k) m[k] = rw.m[3 * k * NS + o];
+        }
+    };
+    auto pair = [&](const HalfQ<R>& qi, const R mi[3], const HalfQ<R>& qj, const R mj[3], R F[5]) {
+        if constexpr (CURV) {
+            const R nv[3] = {mi[0] + mj[0], mi[1] + mj[1], mi[2] + mj[2]};
+            ch_pair_n<R, LM>(qi, qj, nv, cst, F);
+        } else {
+            ch_pair_axis<R, LM>(qi, qj, cst, F);
+        }
+    };
+    // the flux that the previous lane evaluated (towards this lane's nodes)
+    auto from_prev = [&](const R F[5], R G[5]) {
+#pragma unroll
+        for (int s = 0; s < 5; ++s) G[s] = __shfl_sync(0xffffffffu, F[s], prev);
+    };
+    auto add = [&](R a[5], R c, const R F[5]) {
+#pragma unroll
+        for (int s = 0; s < 5; ++s) a[s] += c * F[s];
+    };
+#pragma unroll
+    for (int e = 0; e < NPL; ++e)
+#pragma unroll
+        for (int s = 0; s < 5; ++s) acc[e][s] = R(0);
+    if constexpr (NPL == 2) {
+        // this lane's nodes i0, i1; the next lane's j0, j1; the previous lane's h0, h1. A node adds its
+        // pairs in the order (i, i+1), (i-1, i), (i, i+2), (i-2, i), ..., opposite node last
+        const int i0 = 2 * pos, i1 = i0 + 1;
+        const int j0 = pos + 1 < H ? i0 + 2 : 0, j1 = j0 + 1;
+        const int h0 = pos > 0 ? i0 - 2 : N1 - 2, h1 = h0 + 1;
+        const R* c0 = sS + i0 * N1;
+        const R* c1 = sS + i1 * N1;
+        R* a0 = acc[0];
+        R* a1 = acc[NPL - 1];
+        HalfQ<R> q0, q1;
+        R m0[3], m1[3];
+        node(i0, q0, m0);
+        node(i1, q1, m1);
+        R F[5], G[5];
+        if constexpr (N1 == 2) {
+            pair(q0, m0, q1, m1, F);
+            add(a0, c0[i1], F);
+            add(a1, c1[i0], F);
+        } else if constexpr (N1 == 4) {
+            HalfQ<R> qj;
+            R mj[3], E[5];
+            pair(q0, m0, q1, m1, F);            // k = 1
+            add(a0, c0[i1], F);
+            node(j0, qj, mj);
+            pair(q1, m1, qj, mj, E);
+            from_prev(E, G);
+            add(a0, c0[h1], G);
+            add(a1, c1[j0], E);
+            add(a1, c1[i0], F);
+            // k = 2: the opposite pairs (0, 2) and (1, 3), one on each of the two lanes: lane 0's first
+            // nodes, lane 1's second nodes
+            HalfQ<R> qa = pos == 0 ? q0 : q1, qb;
+            R ma[3], mb[3];
+            if constexpr (CURV) {
+#pragma unroll
+                for (int e = 0; e < 3; ++e) ma[e] = pos == 0 ? m0[e] : m1[e];
+            }
+            node(pos == 0 ? j0 : j1, qb, mb);
+            pair(qa, ma, qb, mb, F);
+            from_prev(F, G);
+            const R ce = c0[j0], cg = c1[j1];
+#pragma unroll
+            for (int s = 0; s < 5; ++s) {
+                const R x = pos == 0 ? F[s] : G[s], y = pos == 0 ? G[s] : F[s];
+                a0[s] += ce * x;
+                a1[s] += cg * y;
+            }
+        } else {
+            static_assert(N1 == 6 || N1 == 4 || N1 == 2, "even lines of 2, 4 or 6 nodes");
+            HalfQ<R> q2;
+            R m2[3], E[5];
+            pair(q0, m0, q1, m1, F);            // k = 1
+            add(a0, c0[i1], F);
+            node(j0, q2, m2);
+            pair(q1, m1, q2, m2, E);
+            from_prev(E, G);
+            add(a0, c0[h1], G);
+            add(a1, c1[j0], E);
+            add(a1, c1[i0], F);
+            pair(q0, m0, q2, m2, F);            // k = 2
+            from_prev(F, G);
+            add(a0, c0[j0], F);
+            add(a0, c0[h0], G);
+            node(j1, q2, m2);
+            pair(q1, m1, q2, m2, F);
+            from_prev(F, G);
+            add(a1, c1[j1], F);
+            add(a1, c1[h1], G);
+            pair(q0, m0, q2, m2, F);            // k = 3
+            from_prev(F, G);
+            add(a0, c0[j1], F);
+            add(a1, c1[h0], G);
+        }
+    } else {
+        // one node per lane: pair (i, i + k) on lane i, k = 1 .. (N1 - 1) / 2
+        HalfQ<R> qi;
+        R mi[3];
+        node(pos, qi, mi);
+#pragma unroll
+        for (int k = 1; k <= N1 / 2; ++k) {
+            const int jp = pos + k < N1 ? pos + k : pos + k - N1, jm = pos - k >= 0 ? pos - k : pos - k + N1;
+            HalfQ<R> qj;
+            R mj[3], F[5];
+            node(jp, qj, mj);
+            pair(qi, mi, qj, mj, F);
+            const R cj = sS[pos * N1 + jp], cr = sS[pos * N1 + jm];
+#pragma unroll
+            for (int s = 0; s < 5; ++s) {
+                const R g = __shfl_sync(0xffffffffu, F[s], jm * SPW + seg);
+                acc[0][s] += cj * F[s];
+                acc[0][s] += cr * g;
+            }
+        }
+    }
 }
 
 // The five DOFs of one node in a Butcher RK stage: the running sum, u_{n+1} and the next stage's input
@@ -292,7 +435,6 @@ __device__ __forceinline__ void line_tile(const StageArgs& a, LineShared<CPC>& s
         const int lineid = (tid >> 5) * L::SPW + seg;
         const bool lvalid = lane < H * L::SPW && lineid < CPC * NF;   // (idle lanes run along on line 0)
         const int lc = lvalid ? lineid / NF : 0, line = lvalid ? lineid - lc * NF : 0;
-        const int prev = (pos == 0 ? H - 1 : pos - 1) * L::SPW + seg;
         const R* Qc = sQ + lc * NQ * NS;
         const R* Lc = sL + lc * 2 * NS;
         R* Ac = sA + lc * 5 * NS;
@@ -305,143 +447,17 @@ __device__ __forceinline__ void line_tile(const StageArgs& a, LineShared<CPC>& s
                 const int base = d == 0 ? N1 * la + ZP * lb : d == 1 ? la + ZP * lb : la + N1 * lb;
                 const int d1 = CURV ? 0 : d, d2 = CURV ? 1 : d == 2 ? 0 : d + 1, d3 = CURV ? 2 : d == 0 ? 2 : d - 1;
                 const int r1 = (1 + d1) * NS, r2 = (1 + d2) * NS, r3 = (1 + d3) * NS;
-                auto node = [&](int i, HalfQ<R>& q, R m[3]) {
-                    const int o = base + i * st;
-                    line_q<R, NS>(Qc, o, r1, r2, r3, q);
-                    if constexpr (LM == LOG_STORED) { q.la = Lc[o]; q.lb = Lc[NS + o]; }
-                    if constexpr (CURV) {
+                R acc[NPL][5];
+                line_pairs<R, N1, NS, CURV, LM>(LineRows<R>{Qc, Qc + 6 * NS, Lc, Qc + (8 + d) * NS, r1, r2, r3}, base, st,
+                                                pos, seg, sS, cst, acc);
+                if (d > 0) __syncthreads();   // the previous direction's terms are in place
+                if (lvalid) {
+                    const int row[5] = {0, r1, r2, r3, 4 * NS};
 #pragma unroll
-                        for (int k = 0; k < 3; ++k) m[k] = Qc[(8 + 3 * k + d) * NS + o];
-                    }
-                };
-                auto pair = [&](const HalfQ<R>& qi, const R mi[3], const HalfQ<R>& qj, const R mj[3], R F[5]) {
-                    if constexpr (CURV) {
-                        const R nv[3] = {mi[0] + mj[0], mi[1] + mj[1], mi[2] + mj[2]};
-                        ch_pair_n<R, LM>(qi, qj, nv, cst, F);
-                    } else {
-                        ch_pair_axis<R, LM>(qi, qj, cst, F);
-                    }
-                };
-                // the flux that the previous lane evaluated (towards this lane's nodes)
-                auto from_prev = [&](const R F[5], R G[5]) {
+                    for (int e = 0; e < NPL; ++e) {
+                        R* A0 = Ac + base + (NPL * pos + e) * st;
 #pragma unroll
-                    for (int s = 0; s < 5; ++s) G[s] = __shfl_sync(0xffffffffu, F[s], prev);
-                };
-                auto add = [&](R acc[5], R c, const R F[5]) {
-#pragma unroll
-                    for (int s = 0; s < 5; ++s) acc[s] += c * F[s];
-                };
-                if constexpr (NPL == 2) {
-                    // this lane's nodes i0, i1; the next lane's j0, j1; the previous lane's h0, h1. A node adds
-                    // its pairs in the order (i, i+1), (i-1, i), (i, i+2), (i-2, i), ..., opposite node last
-                    const int i0 = 2 * pos, i1 = i0 + 1;
-                    const int j0 = pos + 1 < H ? i0 + 2 : 0, j1 = j0 + 1;
-                    const int h0 = pos > 0 ? i0 - 2 : N1 - 2, h1 = h0 + 1;
-                    const R* c0 = sS + i0 * N1;
-                    const R* c1 = sS + i1 * N1;
-                    R a0[5] = {R(0), R(0), R(0), R(0), R(0)}, a1[5] = {R(0), R(0), R(0), R(0), R(0)};
-                    HalfQ<R> q0, q1;
-                    R m0[3], m1[3];
-                    node(i0, q0, m0);
-                    node(i1, q1, m1);
-                    R F[5], G[5];
-                    if constexpr (N1 == 2) {
-                        pair(q0, m0, q1, m1, F);
-                        add(a0, c0[i1], F);
-                        add(a1, c1[i0], F);
-                    } else if constexpr (N1 == 4) {
-                        HalfQ<R> qj;
-                        R mj[3], E[5];
-                        pair(q0, m0, q1, m1, F);            // k = 1
-                        add(a0, c0[i1], F);
-                        node(j0, qj, mj);
-                        pair(q1, m1, qj, mj, E);
-                        from_prev(E, G);
-                        add(a0, c0[h1], G);
-                        add(a1, c1[j0], E);
-                        add(a1, c1[i0], F);
-                        // k = 2: the opposite pairs (0, 2) and (1, 3), one on each of the two lanes: lane 0's first
-                        // nodes, lane 1's second nodes
-                        HalfQ<R> qa = pos == 0 ? q0 : q1, qb;
-                        R ma[3], mb[3];
-                        if constexpr (CURV) {
-#pragma unroll
-                            for (int e = 0; e < 3; ++e) ma[e] = pos == 0 ? m0[e] : m1[e];
-                        }
-                        node(pos == 0 ? j0 : j1, qb, mb);
-                        pair(qa, ma, qb, mb, F);
-                        from_prev(F, G);
-                        const R ce = c0[j0], cg = c1[j1];
-#pragma unroll
-                        for (int s = 0; s < 5; ++s) {
-                            const R x = pos == 0 ? F[s] : G[s], y = pos == 0 ? G[s] : F[s];
-                            a0[s] += ce * x;
-                            a1[s] += cg * y;
-                        }
-                    } else {
-                        static_assert(N1 == 6 || N1 == 4 || N1 == 2, "even lines of 2, 4 or 6 nodes");
-                        HalfQ<R> q2;
-                        R m2[3], E[5];
-                        pair(q0, m0, q1, m1, F);            // k = 1
-                        add(a0, c0[i1], F);
-                        node(j0, q2, m2);
-                        pair(q1, m1, q2, m2, E);
-                        from_prev(E, G);
-                        add(a0, c0[h1], G);
-                        add(a1, c1[j0], E);
-                        add(a1, c1[i0], F);
-                        pair(q0, m0, q2, m2, F);            // k = 2
-                        from_prev(F, G);
-                        add(a0, c0[j0], F);
-                        add(a0, c0[h0], G);
-                        node(j1, q2, m2);
-                        pair(q1, m1, q2, m2, F);
-                        from_prev(F, G);
-                        add(a1, c1[j1], F);
-                        add(a1, c1[h1], G);
-                        pair(q0, m0, q2, m2, F);            // k = 3
-                        from_prev(F, G);
-                        add(a0, c0[j1], F);
-                        add(a1, c1[h0], G);
-                    }
-                    if (d > 0) __syncthreads();   // the previous direction's terms are in place
-                    if (lvalid) {
-                        R* A0 = Ac + base + i0 * st;
-                        R* A1 = A0 + st;
-                        const int row[5] = {0, r1, r2, r3, 4 * NS};
-#pragma unroll
-                        for (int s = 0; s < 5; ++s) {
-                            A0[row[s]] = d == 0 ? a0[s] : A0[row[s]] + a0[s];
-                            A1[row[s]] = d == 0 ? a1[s] : A1[row[s]] + a1[s];
-                        }
-                    }
-                } else {
-                    // one node per lane: pair (i, i + k) on lane i, k = 1 .. (N1 - 1) / 2
-                    R ac[5] = {R(0), R(0), R(0), R(0), R(0)};
-                    HalfQ<R> qi;
-                    R mi[3];
-                    node(pos, qi, mi);
-#pragma unroll
-                    for (int k = 1; k <= N1 / 2; ++k) {
-                        const int jp = pos + k < N1 ? pos + k : pos + k - N1, jm = pos - k >= 0 ? pos - k : pos - k + N1;
-                        HalfQ<R> qj;
-                        R mj[3], F[5];
-                        node(jp, qj, mj);
-                        pair(qi, mi, qj, mj, F);
-                        const R cj = sS[pos * N1 + jp], cr = sS[pos * N1 + jm];
-#pragma unroll
-                        for (int s = 0; s < 5; ++s) {
-                            const R g = __shfl_sync(0xffffffffu, F[s], jm * L::SPW + seg);
-                            ac[s] += cj * F[s];
-                            ac[s] += cr * g;
-                        }
-                    }
-                    if (d > 0) __syncthreads();
-                    if (lvalid) {
-                        R* A0 = Ac + base + pos * st;
-                        const int row[5] = {0, r1, r2, r3, 4 * NS};
-#pragma unroll
-                        for (int s = 0; s < 5; ++s) A0[row[s]] = d == 0 ? ac[s] : A0[row[s]] + ac[s];
+                        for (int s = 0; s < 5; ++s) A0[row[s]] = d == 0 ? acc[e][s] : A0[row[s]] + acc[e][s];
                     }
                 }
             }
