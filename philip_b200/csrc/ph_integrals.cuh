@@ -349,137 +349,173 @@ __global__ void integrals_kernel(const double* __restrict__ U, const double* __r
     }
 }
 
-// Kinetic energy, enstrophy and wave speed on affine cells (the integrals_kernel's partials
-// without FULL) with the y-contraction hoisted out of the point loop: the x- and then the
-// y-contracted values (and x-, y-derivatives of the four fields whose gradient the enstrophy
-// needs) of all columns are built once per cell in shared memory, so a cubature point only
-// contracts along z (4 N1-term sums per field instead of N1 (3 N1 + 4)). Each point's values
-// are the same products summed in the same order as in integrals_kernel. Used while two CTAs
-// fit an SM (p <= 3: 82 KB at p = 3): 2.5 ms against 3.9 ms per evaluation at 32^3 cells,
-// p = 3 on B200; at p = 5 (178 KB, one CTA per SM) it was slower than integrals_kernel.
-constexpr int AFF_THREADS = 256;
-template <int N1> __host__ __device__ constexpr size_t integrals_affine_smem_bytes() {
-    constexpr int NE = N1 + 10;
-    return sizeof(double) * (5 * N1 * N1 * N1 + 2 * N1 * N1 * NE + 13 * N1 * NE * NE);
-}
-template <int N1> __host__ __device__ constexpr bool integrals_affine_fits() {
-    return integrals_affine_smem_bytes<N1>() <= 100 * 1024;
-}
+// Kinetic energy, enstrophy and wave speed on affine cells (the integrals_kernel's partials without FULL).
+// One thread per column of cubature points: it contracts the x-contracted fields along y once, into
+// registers, and walks z. Only what the three integrals need is carried: the values of the five
+// fields, the x-derivatives of rho, m_y, m_z, the y-derivatives of rho, m_x, m_z and (from the values) the
+// z-derivatives of rho, m_x, m_y. Gauss points and solution nodes are symmetric about the cell's
+// centre, so the column is held as even and odd halves and two mirrored points share their sums:
+// 4 operations per field and point at N1 = 6 instead of 6. The factors 1 / h and the cell's volume
+// are taken out of the sums; the wave speed is compared squared (one root per point).
+// Bound by FP64 operations of few warps with much independent work. A step of 16^3 cells of p = 5 with its
+// integrals takes 1.02 ms where the field-by-field contraction at every point took 1.30.
+template <int N1> struct IntegralsAffine {
+    static constexpr int NE = N1 + 10, NP = N1 * N1 * N1, NT2 = N1 * N1 * NE;
+    static constexpr int NT = (NE * NE + 31) / 32 * 32;
+    static constexpr int KE = (N1 + 1) / 2, KO = N1 / 2, QH = (NE + 1) / 2;   // even / odd halves, mirrored point pairs
+    static constexpr int oT0 = 5 * NP, oT1 = oT0 + 5 * NT2, total = oT1 + 3 * NT2;
+    static constexpr size_t bytes = (size_t)total * sizeof(double);
+};
 
 template <int N1>
-__global__ void __launch_bounds__(AFF_THREADS)
+__global__ void __launch_bounds__(IntegralsAffine<N1>::NT)
 integrals_affine_kernel(const double* __restrict__ U, const IntegralTab* tab, int nc, IntegralConst ic,
                         double* __restrict__ partial) {
-    constexpr int NE = N1 + 10;
-    constexpr int NP = N1 * N1 * N1;
-    constexpr int NT2 = N1 * N1 * NE;    // x-contracted entries of one field
-    constexpr int NY = N1 * NE * NE;     // x- and y-contracted entries of one field
+    using L = IntegralsAffine<N1>;
+    constexpr int NE = L::NE, NP = L::NP, NT2 = L::NT2, NT = L::NT, KE = L::KE, KO = L::KO, QH = L::QH;
     __shared__ double sB[NE * N1], sdB[NE * N1], sw[NE];
+    // even / odd parts of B and dB in z: [pair q][k]
+    __shared__ double sE[QH * KE], sO[QH * (KO > 0 ? KO : 1)], sdE[QH * KE], sdO[QH * (KO > 0 ? KO : 1)];
     __shared__ double red[3][32];
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double* sU = reinterpret_cast<double*>(smem_raw);   // [5][NP]
-    double* sTv = sU + 5 * NP;                          // [(k*N1 + j)*NE + qx], one field at a time
-    double* sTx = sTv + NT2;
-    // rows 0-4: values of the five fields; 5-8: x-derivatives and 9-12: y-derivatives of
-    // density and momentum; each row [k][qy*NE + qx]
-    double* sY = sTx + NT2;
-    const int cell = blockIdx.x;
-    const int tid = threadIdx.x;
-    for (int i = tid; i < NE * N1; i += AFF_THREADS) { sB[i] = tab->B[i]; sdB[i] = tab->dB[i]; }
-    for (int i = tid; i < NE; i += AFF_THREADS) sw[i] = tab->w[i];
-    for (int i = tid; i < 5 * NP; i += AFF_THREADS) sU[i] = U[(size_t)cell * 5 * NP + i];
+    double* sT0 = sU + L::oT0;                          // [s][(k*N1 + j)*NE + qx] values
+    double* sT1 = sU + L::oT1;                          // x-derivatives of rho, m_y, m_z
+    const int cell = blockIdx.x, tid = threadIdx.x;
+    for (int i = tid; i < NE * N1; i += NT) { sB[i] = tab->B[i]; sdB[i] = tab->dB[i]; }
+    for (int i = tid; i < NE; i += NT) sw[i] = tab->w[i];
+    for (int i = tid; i < 5 * NP; i += NT) sU[i] = U[(size_t)cell * 5 * NP + i];
     __syncthreads();
-    for (int f = 0; f < 5; ++f) {
-        for (int i = tid; i < NT2; i += AFF_THREADS) {
-            const int qx = i % NE, kj = i / NE;
-            double v = 0.0, dv = 0.0;
-            for (int a = 0; a < N1; ++a) {
-                const double u = sU[f * NP + kj * N1 + a];
-                v += sB[qx * N1 + a] * u;
-                dv += sdB[qx * N1 + a] * u;
-            }
-            sTv[i] = v;
-            sTx[i] = dv;
+    for (int i = tid; i < QH * KE; i += NT) {
+        const int q = i / KE, k = i - q * KE, m = N1 - 1 - k;
+        const double f = k == m ? 0.5 : 1.0;   // the middle node is its own mirror
+        sE[i] = f * 0.5 * (sB[q * N1 + k] + sB[q * N1 + m]);
+        sdE[i] = f * 0.5 * (sdB[q * N1 + k] + sdB[q * N1 + m]);
+        if (k < KO) {
+            sO[q * KO + k] = 0.5 * (sB[q * N1 + k] - sB[q * N1 + m]);
+            sdO[q * KO + k] = 0.5 * (sdB[q * N1 + k] - sdB[q * N1 + m]);
         }
-        __syncthreads();
-        for (int i = tid; i < NY; i += AFF_THREADS) {
-            const int qx = i % NE, qy = (i / NE) % NE, k = i / (NE * NE);
-            double a0 = 0.0, a1 = 0.0, a2 = 0.0;
-#pragma unroll
-            for (int j = 0; j < N1; ++j) {
-                const double t0 = sTv[(k * N1 + j) * NE + qx];
-                const double t1 = sTx[(k * N1 + j) * NE + qx];
-                a0 += sB[qy * N1 + j] * t0;
-                a1 += sB[qy * N1 + j] * t1;
-                a2 += sdB[qy * N1 + j] * t0;
-            }
-            sY[f * NY + i] = a0;
-            if (f < 4) { sY[(5 + f) * NY + i] = a1; sY[(9 + f) * NY + i] = a2; }
-        }
-        __syncthreads();
     }
-    const double inv_h = 1.0 / ic.h, detj = ic.h * ic.h * ic.h;
+    for (int i = tid; i < 5 * NT2; i += NT) {
+        const int qx = i % NE, kj = (i / NE) % (N1 * N1), s = i / NT2;
+        const double* u = sU + s * NP + kj * N1;
+        double v = 0.0, dv = 0.0;
+#pragma unroll
+        for (int a = 0; a < N1; ++a) { v += sB[qx * N1 + a] * u[a]; dv += sdB[qx * N1 + a] * u[a]; }
+        sT0[i] = v;
+        if (s != 1 && s != 4) sT1[(s == 0 ? 0 : s - 1) * NT2 + i - s * NT2] = dv;
+    }
+    __syncthreads();
     const double gam = ic.gam, gm1 = ic.gm1;
-    double ke = 0.0, ens = 0.0, wave = 0.0;
-    for (int pt = tid; pt < NE * NE * NE; pt += AFF_THREADS) {
-        const int col = pt % (NE * NE), qz = pt / (NE * NE);
-        const int qx = col % NE, qy = col / NE;
-        double u[5], g[4][3];
+    double ke = 0.0, en = 0.0, w2 = 0.0;
+    if (tid < NE * NE) {
+        const int qx = tid % NE, qy = tid / NE;
+        // even and odd parts along z of: 0-4 the values, 5-7 d/dx of rho, m_y, m_z, 8-10 d/dy of rho, m_x, m_z
+        double ev[11][KE], od[11][KO > 0 ? KO : 1];
 #pragma unroll
-        for (int f = 0; f < 5; ++f) {
-            double v = 0.0, gx = 0.0, gy = 0.0, gz = 0.0;
+        for (int f = 0; f < 11; ++f) {
+            const double* t = f < 5 ? sT0 + f * NT2 : f < 8 ? sT1 + (f - 5) * NT2
+                                                            : sT0 + (f == 8 ? 0 : f == 9 ? 1 : 3) * NT2;
+            const double* c = (f < 8 ? sB : sdB) + qy * N1;
 #pragma unroll
-            for (int k = 0; k < N1; ++k) {
-                const double b = sB[qz * N1 + k], db = sdB[qz * N1 + k];
-                const double a0 = sY[f * NY + k * NE * NE + col];
-                if (f < 4) {
-                    const double a1 = sY[(5 + f) * NY + k * NE * NE + col];
-                    const double a2 = sY[(9 + f) * NY + k * NE * NE + col];
-                    v += b * a0; gx += b * a1; gy += b * a2; gz += db * a0;
-                } else {
-                    v += b * a0;
+            for (int k = 0; k < KE; ++k) {
+                const int m = N1 - 1 - k;
+                double x = 0.0, y = 0.0;
+#pragma unroll
+                for (int j = 0; j < N1; ++j) {
+                    x += c[j] * t[(k * N1 + j) * NE + qx];
+                    if (m != k) y += c[j] * t[(m * N1 + j) * NE + qx];
                 }
+                if (m == k) y = x;
+                ev[f][k] = x + y;
+                if (k < KO) od[f][k] = x - y;
             }
-            u[f] = v;
-            if (f < 4) { g[f][0] = gx * inv_h; g[f][1] = gy * inv_h; g[f][2] = gz * inv_h; }
         }
-        const double rho = u[0];
-        double v[3], v2 = 0.0;
+#pragma unroll 1
+        for (int q = 0; q < QH; ++q) {
+            // the pair's two points: field f (0-10 as above, 11-13 d/dz of rho, m_x, m_y) at q and at its mirror
+            auto points = [&](int f, double d[2]) {
+                const int r = f < 11 ? f : f - 11;
+                double e = 0.0, o = 0.0;
 #pragma unroll
-        for (int d = 0; d < 3; ++d) { v[d] = u[1 + d] / rho; v2 += v[d] * v[d]; }
-        double gv[3][3];
+                for (int k = 0; k < KE; ++k) e += (f < 11 ? sE : sdE)[q * KE + k] * ev[r][k];
 #pragma unroll
-        for (int a = 0; a < 3; ++a)
+                for (int k = 0; k < KO; ++k) o += (f < 11 ? sO : sdO)[q * KO + k] * od[r][k];
+                d[0] = e + o;
+                d[1] = f < 11 ? e - o : o - e;
+            };
+            double rho[2], v[3][2], en_[2], om[3][2], d[2];
+            points(0, rho); points(1, v[0]); points(2, v[1]); points(3, v[2]); points(4, en_);
+            double ir[2], vv[2];
 #pragma unroll
-            for (int d = 0; d < 3; ++d) gv[a][d] = (g[1 + a][d] - v[a] * g[0][d]) / rho;
-        const double o0 = gv[2][1] - gv[1][2], o1 = gv[0][2] - gv[2][0], o2 = gv[1][0] - gv[0][1];
-        const double wt = sw[qx] * sw[qy] * sw[qz] * detj;
-        ke += 0.5 * rho * v2 * wt;
-        ens += 0.5 * rho * (o0 * o0 + o1 * o1 + o2 * o2) * wt;
-        const double p = gm1 * (u[4] - 0.5 * rho * v2);
-        const double c = sqrt(p * gam / rho);
-        const double ws = sqrt(v2) + c;
-        wave = ws > wave ? ws : wave;
+            for (int m = 0; m < 2; ++m) {
+                ir[m] = qrcp<double>(rho[m]);
+#pragma unroll
+                for (int c = 0; c < 3; ++c) v[c][m] *= ir[m];
+                vv[m] = v[0][m] * v[0][m] + v[1][m] * v[1][m] + v[2][m] * v[2][m];
+            }
+            // om: rho times the vorticity (times h), derivative by derivative
+            points(5, d);    // d rho / dx
+#pragma unroll
+            for (int m = 0; m < 2; ++m) { om[1][m] = v[2][m] * d[m]; om[2][m] = -(v[1][m] * d[m]); }
+            points(6, d);    // d m_y / dx
+#pragma unroll
+            for (int m = 0; m < 2; ++m) om[2][m] += d[m];
+            points(7, d);    // d m_z / dx
+#pragma unroll
+            for (int m = 0; m < 2; ++m) om[1][m] -= d[m];
+            points(8, d);    // d rho / dy
+#pragma unroll
+            for (int m = 0; m < 2; ++m) { om[0][m] = -(v[2][m] * d[m]); om[2][m] += v[0][m] * d[m]; }
+            points(9, d);    // d m_x / dy
+#pragma unroll
+            for (int m = 0; m < 2; ++m) om[2][m] -= d[m];
+            points(10, d);   // d m_z / dy
+#pragma unroll
+            for (int m = 0; m < 2; ++m) om[0][m] += d[m];
+            points(11, d);   // d rho / dz
+#pragma unroll
+            for (int m = 0; m < 2; ++m) { om[0][m] += v[1][m] * d[m]; om[1][m] -= v[0][m] * d[m]; }
+            points(12, d);   // d m_x / dz
+#pragma unroll
+            for (int m = 0; m < 2; ++m) om[1][m] += d[m];
+            points(13, d);   // d m_y / dz
+#pragma unroll
+            for (int m = 0; m < 2; ++m) om[0][m] -= d[m];
+            const double wz = sw[q];
+#pragma unroll
+            for (int m = 0; m < 2; ++m) {
+                if (m && 2 * q + 1 == NE) continue;   // (the centre is its own mirror)
+                ke += wz * (rho[m] * vv[m]);
+                en += wz * ((om[0][m] * om[0][m] + om[1][m] * om[1][m] + om[2][m] * om[2][m]) * ir[m]);
+                const double p = gm1 * (en_[m] - 0.5 * rho[m] * vv[m]), cc = gam * p * ir[m];
+                const double s2 = (vv[m] + cc) + 2.0 * sqrt(vv[m] * cc);   // (|v| + c)^2
+                w2 = s2 > w2 ? s2 : w2;
+            }
+        }
+        const double wxy = 0.5 * (sw[qx] * sw[qy]);
+        ke *= wxy * (ic.h * ic.h * ic.h);
+        en *= wxy * ic.h;   // h^3 / h^2
     }
+    // block reduction in a fixed order (warp shuffles, then the warps in order)
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         ke += __shfl_down_sync(0xffffffffu, ke, o);
-        ens += __shfl_down_sync(0xffffffffu, ens, o);
-        const double wo = __shfl_down_sync(0xffffffffu, wave, o);
-        wave = wo > wave ? wo : wave;
+        en += __shfl_down_sync(0xffffffffu, en, o);
+        const double wo = __shfl_down_sync(0xffffffffu, w2, o);
+        w2 = wo > w2 ? wo : w2;
     }
-    const int warp = tid >> 5, lane = tid & 31;
-    if (lane == 0) { red[0][warp] = ke; red[1][warp] = ens; red[2][warp] = wave; }
+    if ((tid & 31) == 0) { red[0][tid >> 5] = ke; red[1][tid >> 5] = en; red[2][tid >> 5] = w2; }
     __syncthreads();
     if (tid == 0) {
         double a0 = 0.0, a1 = 0.0, a2 = 0.0;
-        for (int w = 0; w < AFF_THREADS / 32; ++w) {
+        for (int w = 0; w < NT / 32; ++w) {
             a0 += red[0][w]; a1 += red[1][w];
             a2 = red[2][w] > a2 ? red[2][w] : a2;
         }
-        partial[3 * (size_t)cell + 0] = a0;
-        partial[3 * (size_t)cell + 1] = a1;
-        partial[3 * (size_t)cell + 2] = a2;
+        partial[(size_t)3 * cell] = a0;
+        partial[(size_t)3 * cell + 1] = a1;
+        partial[(size_t)3 * cell + 2] = sqrt(a2);
     }
 }
 
