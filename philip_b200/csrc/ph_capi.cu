@@ -560,7 +560,7 @@ int build_gl_operators(const ph_params* prm, ph::GlTab& t, ph::OpTab& ops) {
             }
     std::vector<double> Mi;
     if (!mat_inv(M, nd, Mi)) return fail(PH_ERR_INVALID, "singular mass matrix");
-    // projection M^-1 chi^T W (nd x nq), then P = chi proj and the face rows chis proj
+    // projection M^-1 chi^T W (nd x nq), then P = chi proj
     std::vector<double> proj((size_t)nd * nq, 0.0);
     for (int i = 0; i < nd; ++i)
         for (int q = 0; q < nq; ++q) {
@@ -573,12 +573,6 @@ int build_gl_operators(const ph_params* prm, ph::GlTab& t, ph::OpTab& ops) {
             double v = 0.0;
             for (int i = 0; i < nd; ++i) v += chi[a * nd + i] * proj[i * nq + q];
             t.P[a * nq + q] = v;
-        }
-    for (int side = 0; side < 2; ++side)
-        for (int q = 0; q < nq; ++q) {
-            double v = 0.0;
-            for (int i = 0; i < nd; ++i) v += t.chis[side][i] * proj[i * nq + q];
-            t.ps[side][q] = v;
         }
     // FR: D = M^-1 Schi, K = c (D^p)^T M D^p; the auxiliary equation's K_aux takes k for c
     double cfr = 0.0, kaux = 0.0;
@@ -603,17 +597,12 @@ int build_gl_operators(const ph_params* prm, ph::GlTab& t, ph::OpTab& ops) {
     if (!mat_inv(MK, nd, MKi)) return fail(PH_ERR_INVALID, "singular FR mass matrix");
     if (kaux == 0.0) MKai = Mi;
     else if (!mat_inv(MKa, nd, MKai)) return fail(PH_ERR_INVALID, "singular auxiliary FR mass matrix");
-    // (M + K)^-1 folded into the transposed lifts: chi (M + K)^-1 and (M + K)^-1 chis (M + K is symmetric)
+    // (M + K)^-1 folded into the transposed interpolation: chi (M + K)^-1 (M + K is symmetric)
     for (int i = 0; i < nd; ++i) {
         for (int q = 0; q < nq; ++q) {
             double v = 0.0;
             for (int j = 0; j < nd; ++j) v += chi[q * nd + j] * MKi[j * nd + i];
             t.chm[q * nd + i] = v;
-        }
-        for (int side = 0; side < 2; ++side) {
-            double v = 0.0;
-            for (int j = 0; j < nd; ++j) v += MKi[i * nd + j] * t.chis[side][j];
-            t.chms[side][i] = v;
         }
     }
     // chi (M + K_aux)^-1 chi^T (nq x nq): the auxiliary equation's inverse mass seen from the flux

@@ -15,13 +15,13 @@
 //   gl_trace_kernel  the state's face values (chi_s (x) chi (x) chi U) and, for the split form, the
 //                    states of the projected entropy variables at the face nodes and at the volume
 //                    flux nodes (projected once, read by the other two kernels)
-//   gl_aux_kernel    (Navier-Stokes) the lifted gradient q = (M_aux)^-1 [chi^T W D(chi u)
+//   gl_aux_kernel    (Navier-Stokes; gl_aux_line_kernel on affine periodic cells) the lifted gradient q = (M_aux)^-1 [chi^T W D(chi u)
 //                    + face (u* - u) n], kept at the flux nodes, then the viscous volume term
 //                    W div(F_v) at the flux nodes, and per face node F_v(u, q) . n and the face-normal
 //                    volume viscous flux
 //   gl_stage_kernel  volume term (two-point split form with the skew operator on flux-node
 //                    lines, or the conservative divergence), hybrid surface-volume two-point
-//                    terms, numerical fluxes, lifts with (M+K)^-1 folded into their operators and
+//                    terms, numerical fluxes, lifts at the flux nodes, (M+K)^-1 folded into the last passes and
 //                    the RK stage update
 // The face data of a neighbour come from the buffers the earlier kernels wrote, so every
 // face's numerical flux sees the same two states from either side.
@@ -51,11 +51,9 @@ struct GlTab {
     double skew[GL_MAXQ * GL_MAXQ];   // S - S^T, S_ij = sum_q phi_i phi_j' w_q (operators.cpp:1440-1477)
     double wq[GL_MAXQ];               // flux-node weights on [0, 1]
     double P[GL_MAXQ * GL_MAXQ];      // chi M^-1 chi^T W: flux values -> projected -> flux values
-    double ps[2][GL_MAXQ];            // chis[side] M^-1 chi^T W: face value of the projection
     double haux[GL_MAXQ * GL_MAXQ];   // chi (M + K_aux)^-1 chi^T
     double pwa[GL_MAXD * GL_MAXQ];    // (M + K)^-1 chi^T W (nd x nq): the weight-adjusted inverse mass's projection
     double chm[GL_MAXQ * GL_MAXD];    // chi (M + K)^-1 (nq x nd): the transposed lift and the inverse mass in one
-    double chms[2][GL_MAXD];          // (M + K)^-1 chis[side]
 };
 
 // Device buffers of the uncollocated path (per cell, reference units).
@@ -330,123 +328,25 @@ template <int N> __device__ __forceinline__ int gl_line_node(int dn, int q2, int
     return dn == 0 ? (t2c * N + t1c) * N + l : dn == 1 ? (t2c * N + l) * N + t1c : (l * N + t2c) * N + t1c;
 }
 
-// Face values on all six faces of NS cubes of NIN^3 values: for face f (normal dn = f / 2,
-// side f & 1) out[f][s][q2] = sum row[side][i_dn] T[q_t1][i_t1] T[q_t2][i_t2] src[s][i]
-// (the surface interpolation of operators.cpp:355-398 with the face's row along the normal),
-// q2 = q_t2 * NOUT + q_t1. row0 / row1 (NIN values) are read with run-time indices (shared
-// memory); T (NOUT x NIN, a kernel parameter) only with compile-time ones; without HAS_T the
-// tangential operator is the identity (NOUT = NIN). w0: 6 NS NIN^2 values, w1: 6 NS NOUT NIN.
-// Ends with a barrier.
-template <int NT, int NIN, int NOUT, int NS, bool HAS_T>
-__device__ __forceinline__ void gl_face_values(const double* src, int src_ss, const double* row0, const double* row1,
-                                               const double* T, double* w0, double* w1, double* out, int out_fs,
-                                               int out_ss) {
-    constexpr int N2 = NIN * NIN;
-    for (int it = threadIdx.x; it < 6 * NS * N2; it += NT) {   // along the normal: w0[f][s][b * NIN + a]
-        const int f = it / (NS * N2), r = it - f * NS * N2, s = r / N2, ab = r - s * N2;
-        const int a = ab % NIN, b = ab / NIN, dn = f >> 1;
-        const double* rw = (f & 1) ? row1 : row0;
-        const int st = dn == 0 ? 1 : dn == 1 ? NIN : N2;
-        const int base = dn == 0 ? (b * NIN + a) * NIN : dn == 1 ? b * N2 + a : b * NIN + a;
-        const double* ip = src + s * src_ss + base;
-        double v = 0.0;
+// The two end values of a line of flux-node values: the flux-node basis at xi = 0 and 1. The solution
+// basis is interpolated exactly by the flux-node basis (chis[side] = chi^T phis[side]), so a face value of a
+// discrete function is one contraction along the normal of its flux-node values, and a face array is
+// lifted by adding phis[side][l] times it to the flux-node array whose chi^T (x3) follows.
+template <int NQ>
+__device__ __forceinline__ void gl_line_ends(const GlTab& T, const double* ip, int st, double& v0, double& v1) {
+    v0 = v1 = 0.0;
 #pragma unroll
-        for (int l = 0; l < NIN; ++l) v += rw[l] * ip[l * st];
-        if constexpr (HAS_T) w0[it] = v;
-        else out[f * out_fs + s * out_ss + ab] = v;
-    }
-    __syncthreads();
-    if constexpr (HAS_T) {
-        for (int it = threadIdx.x; it < 6 * NS * NIN; it += NT) {   // along t1: w1[f][s][b * NOUT + q1]
-            const double* ip = w0 + it * NIN;
-            double v[NIN];
-#pragma unroll
-            for (int l = 0; l < NIN; ++l) v[l] = ip[l];
-            double* op = w1 + it * NOUT;
-#pragma unroll
-            for (int o = 0; o < NOUT; ++o) {
-                double x = 0.0;
-#pragma unroll
-                for (int l = 0; l < NIN; ++l) x += T[o * NIN + l] * v[l];
-                op[o] = x;
-            }
-        }
-        __syncthreads();
-        for (int it = threadIdx.x; it < 6 * NS * NOUT; it += NT) {   // along t2
-            const int fs = it / NOUT, q1 = it - fs * NOUT, f = fs / NS, s = fs - f * NS;
-            const double* ip = w1 + fs * NOUT * NIN + q1;
-            double v[NIN];
-#pragma unroll
-            for (int l = 0; l < NIN; ++l) v[l] = ip[l * NOUT];
-            double* op = out + f * out_fs + s * out_ss + q1;
-#pragma unroll
-            for (int o = 0; o < NOUT; ++o) {
-                double x = 0.0;
-#pragma unroll
-                for (int l = 0; l < NIN; ++l) x += T[o * NIN + l] * v[l];
-                op[o * NOUT] = x;
-            }
-        }
-        __syncthreads();
+    for (int l = 0; l < NQ; ++l) {
+        const double x = ip[l * st];
+        v0 += T.phis[0][l] * x;
+        v1 += T.phis[1][l] * x;
     }
 }
-
-// The lift of six face arrays into NS cubes of ND^3: dst[s][node] (+)= sum_f row[side][i_dn]
-// sum_{q1,q2} T[q1][i_t1] T[q2][i_t2] face[f][s][q2] (the surface inner products of
-// operators.cpp:575-636 with the solution basis; T is NQ x ND, a kernel parameter; row0 / row1
-// in shared memory). w0: 6 NS NQ ND, w1: 6 NS ND^2 values. Ends with a barrier.
-template <int NT, int NQ, int ND, int NS>
-__device__ __forceinline__ void gl_lift_faces(const double* face, int face_fs, int face_ss, const double* row0,
-                                              const double* row1, const double* T, double* w0, double* w1, double* dst,
-                                              int dst_ss, double scale) {
-    constexpr int MQ = NQ * NQ, D2 = ND * ND, D3 = D2 * ND;
-    for (int it = threadIdx.x; it < 6 * NS * NQ; it += NT) {   // along t1: w0[f][s][q2][a]
-        const int fs = it / NQ, q2 = it - fs * NQ, f = fs / NS, s = fs - f * NS;
-        const double* ip = face + f * face_fs + s * face_ss + q2 * NQ;
-        double v[NQ];
-#pragma unroll
-        for (int l = 0; l < NQ; ++l) v[l] = ip[l];
-        double* op = w0 + (fs * NQ + q2) * ND;
-#pragma unroll
-        for (int o = 0; o < ND; ++o) {
-            double x = 0.0;
-#pragma unroll
-            for (int l = 0; l < NQ; ++l) x += T[l * ND + o] * v[l];
-            op[o] = x;
-        }
-    }
-    __syncthreads();
-    for (int it = threadIdx.x; it < 6 * NS * ND; it += NT) {   // along t2: w1[f][s][b * ND + a]
-        const int fs = it / ND, a = it - fs * ND;
-        const double* ip = w0 + fs * NQ * ND + a;
-        double v[NQ];
-#pragma unroll
-        for (int l = 0; l < NQ; ++l) v[l] = ip[l * ND];
-        double* op = w1 + fs * D2 + a;
-#pragma unroll
-        for (int o = 0; o < ND; ++o) {
-            double x = 0.0;
-#pragma unroll
-            for (int l = 0; l < NQ; ++l) x += T[l * ND + o] * v[l];
-            op[o * ND] = x;
-        }
-    }
-    __syncthreads();
-    for (int it = threadIdx.x; it < NS * D3; it += NT) {
-        const int s = it / D3, node = it - s * D3;
-        const int c[3] = {node % ND, (node / ND) % ND, node / D2};
-        double* op = dst + s * dst_ss + node;
-#pragma unroll
-        for (int dn = 0; dn < 3; ++dn) {
-            const int t1 = dn == 0 ? 1 : 0, t2 = dn == 2 ? 1 : 2;
-            const int ab = c[t2] * ND + c[t1];
-            const double v = row0[c[dn]] * w1[((2 * dn) * NS + s) * D2 + ab] +
-                             row1[c[dn]] * w1[((2 * dn + 1) * NS + s) * D2 + ab];
-            *op += scale * v;
-        }
-    }
-    __syncthreads();
-    (void)MQ;
+// first node of line `line` (face-node order q2) along direction d and the line's stride
+template <int NQ> __device__ __forceinline__ int gl_line_base(int d, int line, int& st) {
+    const int a = line % NQ, b = line / NQ;
+    st = d == 0 ? 1 : d == 1 ? NQ : NQ * NQ;
+    return d == 0 ? NQ * line : d == 1 ? a + NQ * NQ * b : line;
 }
 
 // Shared-memory copy of the operator table (for the reads with run-time indices).
@@ -461,39 +361,45 @@ __device__ __forceinline__ void gl_load_tab(const GlTab* g, GlTab* s, int nt) {
 // ------------------------------------------------------------------------------------
 template <int ND, int NQ, bool SPLIT>
 struct GlTraceLayout {
-    static constexpr int NT = gl_threads<NQ>();
+    static constexpr int NT = NQ == 6 ? 192 : gl_threads<NQ>();     // 180 lines per pass at NQ = 6
     static constexpr int D3 = ND * ND * ND, Q3 = NQ * NQ * NQ;
-    static constexpr int oTab = 0, nTab = (int)(sizeof(GlTab) / sizeof(double));
-    static constexpr int oU = nTab;                                 // 5 ND^3
-    static constexpr int oQ = oU + 5 * D3;                          // 5 NQ^3 (flux-node values / entropy variables)
-    static constexpr int nW = gl_temp<ND, NQ>();
+    static constexpr int oQ = 0;                                    // 5 NQ^3 (flux-node values / entropy variables)
+    static constexpr int nW = 5 * Q3;
     static constexpr int oW0 = oQ + 5 * Q3, oW1 = oW0 + nW;
     static constexpr int total = oW1 + nW;
     static constexpr size_t bytes = (size_t)total * sizeof(double);
 };
 
 template <int ND, int NQ, bool SPLIT>
-__global__ void __launch_bounds__(gl_threads<NQ>())
+__global__ void __launch_bounds__(GlTraceLayout<ND, NQ, SPLIT>::NT)
 gl_trace_kernel(const StageArgs a, const GlArgs g, const __grid_constant__ GlTab T) {
     using L = GlTraceLayout<ND, NQ, SPLIT>;
-    constexpr int NT = L::NT, D3 = L::D3, Q3 = L::Q3, T1W = gl_t1_width<SPLIT>();
+    constexpr int NT = L::NT, D3 = L::D3, Q3 = L::Q3, NF = NQ * NQ, T1W = gl_t1_width<SPLIT>();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double* sm = reinterpret_cast<double*>(smem_raw);
-    GlTab* tab = reinterpret_cast<GlTab*>(sm + L::oTab);
-    double* sU = sm + L::oU;
     double* sQ = sm + L::oQ;
     double* w0 = sm + L::oW0;
     double* w1 = sm + L::oW1;
     const int cell = a.cell_begin + blockIdx.x;
-    gl_load_tab(g.tab, tab, NT);
-    for (int i = threadIdx.x; i < 5 * D3; i += NT) sU[i] = __ldg(&a.U[(size_t)cell * 5 * D3 + i]);
+    for (int i = threadIdx.x; i < 5 * D3; i += NT) sQ[i] = __ldg(&a.U[(size_t)cell * 5 * D3 + i]);
     __syncthreads();
-    double* out = g.t1 + (size_t)cell * 6 * T1W * NQ * NQ;
-    gl_face_values<NT, ND, NQ, 5, true>(sU, D3, tab->chis[0], tab->chis[1], T.chi, w0, w1, out, T1W * NQ * NQ,
-                                        NQ * NQ);
+    gl_apply3<NT, NQ, ND, 5>(T.chi, sQ, D3, sQ, Q3, w0, w1, 1.0, false);
+    double* out = g.t1 + (size_t)cell * 6 * T1W * NF;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        for (int it = threadIdx.x; it < 5 * NF; it += NT) {
+            const int s = it / NF, line = it - s * NF;
+            int st;
+            const int base = gl_line_base<NQ>(d, line, st);
+            double v0, v1;
+            gl_line_ends<NQ>(T, sQ + s * Q3 + base, st, v0, v1);
+            out[((2 * d) * T1W + s) * NF + line] = v0;
+            out[((2 * d + 1) * T1W + s) * NF + line] = v1;
+        }
+    }
     if constexpr (SPLIT) {
-        gl_apply3<NT, NQ, ND, 5>(T.chi, sU, D3, sQ, Q3, w0, w1, 1.0, false);
         const double gam = a.pc.gam, gm1 = a.pc.gm1;
+        __syncthreads();
         for (int q = threadIdx.x; q < Q3; q += NT) {
             double u[5], v[5];
 #pragma unroll
@@ -503,26 +409,29 @@ gl_trace_kernel(const StageArgs a, const GlArgs g, const __grid_constant__ GlTab
             for (int s = 0; s < 5; ++s) sQ[s * Q3 + q] = v[s];
         }
         __syncthreads();
-        constexpr int NF = NQ * NQ;
-        gl_face_values<NT, NQ, NQ, 5, true>(sQ, Q3, tab->ps[0], tab->ps[1], T.P, w0, w1, w0, 5 * NF, NF);
-        for (int it = threadIdx.x; it < 6 * NF; it += NT) {
-            const int f = it / NF, q2 = it - f * NF;
-            double v[5], u[5];
-#pragma unroll
-            for (int s = 0; s < 5; ++s) v[s] = w0[(f * 5 + s) * NF + q2];
-            gl_cons_from_entropy(v, gam, gm1, u);
-#pragma unroll
-            for (int s = 0; s < 5; ++s) out[(f * T1W + 5 + s) * NF + q2] = u[s];
-        }
-        __syncthreads();
         gl_apply3<NT, NQ, NQ, 5>(T.P, sQ, Q3, sQ, Q3, w0, w1, 1.0, false);
-        for (int q = threadIdx.x; q < Q3; q += NT) {
-            double v[5], u[5];
+        for (int it = threadIdx.x; it < Q3 + 3 * NF; it += NT) {
+            if (it < Q3) {
+                double v[5], u[5];
 #pragma unroll
-            for (int s = 0; s < 5; ++s) v[s] = sQ[s * Q3 + q];
-            gl_cons_from_entropy(v, gam, gm1, u);
+                for (int s = 0; s < 5; ++s) v[s] = sQ[s * Q3 + it];
+                gl_cons_from_entropy(v, gam, gm1, u);
 #pragma unroll
-            for (int s = 0; s < 5; ++s) g.proj[((size_t)cell * 5 + s) * Q3 + q] = u[s];
+                for (int s = 0; s < 5; ++s) g.proj[((size_t)cell * 5 + s) * Q3 + it] = u[s];
+            } else {   // the two face nodes of a line
+                const int d = (it - Q3) / NF, line = (it - Q3) - d * NF;
+                int st;
+                const int base = gl_line_base<NQ>(d, line, st);
+                double v[2][5], u[5];
+#pragma unroll
+                for (int s = 0; s < 5; ++s) gl_line_ends<NQ>(T, sQ + s * Q3 + base, st, v[0][s], v[1][s]);
+#pragma unroll
+                for (int side = 0; side < 2; ++side) {
+                    gl_cons_from_entropy(v[side], gam, gm1, u);
+#pragma unroll
+                    for (int s = 0; s < 5; ++s) out[((2 * d + side) * T1W + 5 + s) * NF + line] = u[s];
+                }
+            }
         }
     }
 }
@@ -810,6 +719,176 @@ gl_aux_kernel(const StageArgs a, const GlArgs g, const __grid_constant__ GlTab T
     }
 }
 
+// The same on affine cells without boundary faces, line by line: the derivative pass adds the weights and
+// the faces' lifts as it writes, a face node's gradient is contracted once for both ends of its line,
+// and each direction's flux lines give the face-normal fluxes at their ends and are replaced by their
+// derivatives (summed as they are stored). gl_aux_kernel, which serves the other cells, is bound by index
+// arithmetic and shared-memory traffic: 136 us at 12^3 cells of p = 5, here 83 us (FP64 pipe 34 % busy,
+// shared memory 50 %, three CTAs per SM by registers). 192 threads at NQ = 6 take the 180 lines of a
+// direction's five rows in one pass.
+template <int ND, int NQ, bool SPLIT>
+struct GlAuxLineLayout {
+    static constexpr int NT = NQ <= 4 ? 64 : NQ == 5 ? 128 : NQ == 6 ? 192 : 256;
+    static constexpr int D3 = ND * ND * ND, Q3 = NQ * NQ * NQ, NF = NQ * NQ;
+    static constexpr int oQ = 0;                          // 5 NQ^3 state at the flux nodes
+    static constexpr int oG = oQ + 5 * Q3;                // 15 NQ^3 lifted gradient, later flux rows d * 4 + k
+    static constexpr int nR = SPLIT && 12 * Q3 > 30 * NF ? 12 * Q3 : 30 * NF;
+    static constexpr int oR = oG + 15 * Q3;               // [d][s][2][NF] face terms, later (split) the state's own flux
+    static constexpr int total = oR + nR;
+    static constexpr size_t bytes = (size_t)total * sizeof(double);
+    // CTAs per SM asked of the register allocator (96 registers at NQ = 6)
+    static constexpr int MINB = NQ <= 4 ? 8 : NQ == 5 ? 4 : NQ == 6 ? 3 : 2;
+};
+
+template <int ND, int NQ, bool SPLIT>
+__global__ void __launch_bounds__(GlAuxLineLayout<ND, NQ, SPLIT>::NT, GlAuxLineLayout<ND, NQ, SPLIT>::MINB)
+gl_aux_line_kernel(const StageArgs a, const GlArgs g, const __grid_constant__ GlTab T) {
+    using L = GlAuxLineLayout<ND, NQ, SPLIT>;
+    constexpr int NT = L::NT, D3 = L::D3, Q3 = L::Q3, NF = L::NF, T1W = gl_t1_width<SPLIT>();
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ double wq[NQ];
+    double* sm = reinterpret_cast<double*>(smem_raw);
+    double* sQ = sm + L::oQ;
+    double* sG = sm + L::oG;
+    double* sR = sm + L::oR;
+    const int cell = a.tiles ? __ldg(&a.tiles[blockIdx.x]) : a.cell_begin + (int)blockIdx.x;
+    const int tid = threadIdx.x;
+    Cst<double> cst; cst.load(a.pc);
+    const int ucv = a.pc.use_const_visc;
+    if (tid < NQ) wq[tid] = g.tab->wq[tid];
+    for (int i = tid; i < 5 * D3; i += NT) sQ[i] = __ldg(&a.U[(size_t)cell * 5 * D3 + i]);
+    // faces: (u* - u) n at the two ends of every line
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+        for (int it = tid; it < 10 * NF; it += NT) {
+            const int s = it / (2 * NF), r = it - s * 2 * NF, side = r / NF, q2 = r - side * NF, f = 2 * d + side;
+            const int cn = __ldg(&a.nbr[cell * 6 + f]);
+            const double uo = __ldg(&g.t1[(((size_t)cell * 6 + f) * T1W + s) * NF + q2]);
+            const double ue = __ldg(&g.t1[(((size_t)cn * 6 + (f ^ 1)) * T1W + s) * NF + q2]);
+            sR[d * 10 * NF + it] = (0.5 * (uo + ue) - uo) * (side ? 1.0 : -1.0);
+        }
+    __syncthreads();
+    gl_apply3<NT, NQ, ND, 5>(T.chi, sQ, D3, sQ, Q3, sG, sG + 5 * Q3, 1.0, false);
+    // W D_d u + the faces' lifts, into row d * 5 + s: one thread per line
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+        for (int it = tid; it < 5 * NF; it += NT) {
+            const int s = it / NF, line = it - s * NF;
+            int st;
+            const int base = gl_line_base<NQ>(d, line, st);
+            const double* ip = sQ + s * Q3 + base;
+            double* op = sG + (d * 5 + s) * Q3 + base;
+            const double f0 = sR[d * 10 * NF + s * 2 * NF + line], f1 = sR[d * 10 * NF + s * 2 * NF + NF + line];
+            const double wab = wq[line % NQ] * wq[line / NQ];
+            double v[NQ];
+#pragma unroll
+            for (int l = 0; l < NQ; ++l) v[l] = ip[l * st];
+#pragma unroll
+            for (int o = 0; o < NQ; ++o) {
+                double x = 0.0;
+#pragma unroll
+                for (int l = 0; l < NQ; ++l) x += T.dphi[o * NQ + l] * v[l];
+                op[o * st] = wab * (T.wq[o] * x + (T.phis[0][o] * f0 + T.phis[1][o] * f1));
+            }
+        }
+    __syncthreads();
+    gl_line<NT, NQ, NQ, 0, NQ, NQ, NQ, 15>(T.haux, sG, Q3, sG, Q3, 1.0, false);
+    __syncthreads();
+    gl_line<NT, NQ, NQ, 1, NQ, NQ, NQ, 15>(T.haux, sG, Q3, sG, Q3, 1.0, false);
+    __syncthreads();
+    gl_line<NT, NQ, NQ, 2, NQ, NQ, NQ, 15>(T.haux, sG, Q3, sG, Q3, a.inv_h, false);
+    __syncthreads();
+    // per face node of the cell: F_v(u, q) . e_d with the state's and the gradient's face values
+    double* tout = g.t2 + (size_t)cell * 6 * GL_T2W * NF;
+#pragma unroll 1
+    for (int it = tid; it < 3 * NF; it += NT) {
+        const int d = it / NF, line = it - d * NF;
+        int st;
+        const int base = gl_line_base<NQ>(d, line, st);
+        double gq[2][5][3];
+#pragma unroll
+        for (int e = 0; e < 3; ++e)
+#pragma unroll
+            for (int s = 0; s < 5; ++s)
+                gl_line_ends<NQ>(T, sG + (e * 5 + s) * Q3 + base, st, gq[0][s][e], gq[1][s][e]);
+#pragma unroll
+        for (int side = 0; side < 2; ++side) {
+            double r[5], F[3][4];
+#pragma unroll
+            for (int s = 0; s < 5; ++s) r[s] = __ldg(&g.t1[(((size_t)cell * 6 + 2 * d + side) * T1W + s) * NF + line]);
+            viscous_flux<double>(r, gq[side], ucv, cst, F, 7, nullptr);
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                tout[((2 * d + side) * GL_T2W + k) * NF + line] = d == 0 ? F[0][k] : d == 1 ? F[1][k] : F[2][k];
+        }
+    }
+    __syncthreads();   // (the gradient rows are overwritten below)
+    // nodal fluxes: the split form evaluates the volume term at the entropy-projected state
+    // (strong_dg.cpp:1328 before :1392), the face-normal flux with the state itself (:2836-3041)
+#pragma unroll 1
+    for (int q = tid; q < Q3; q += NT) {
+        double u[5], gq[5][3], F[3][4];
+#pragma unroll
+        for (int s = 0; s < 5; ++s) {
+            u[s] = sQ[s * Q3 + q];
+#pragma unroll
+            for (int e = 0; e < 3; ++e) gq[s][e] = sG[(e * 5 + s) * Q3 + q];
+        }
+        viscous_flux<double>(u, gq, ucv, cst, F, 7, nullptr);
+        double* R = (SPLIT ? sR : sG) + q;
+#pragma unroll
+        for (int e = 0; e < 3; ++e)
+#pragma unroll
+            for (int k = 0; k < 4; ++k) R[(e * 4 + k) * Q3] = F[e][k];
+        if constexpr (SPLIT) {
+#pragma unroll
+            for (int s = 0; s < 5; ++s) u[s] = __ldg(&g.proj[((size_t)cell * 5 + s) * Q3 + q]);
+            viscous_flux<double>(u, gq, ucv, cst, F, 7, nullptr);
+#pragma unroll
+            for (int e = 0; e < 3; ++e)
+#pragma unroll
+                for (int k = 0; k < 4; ++k) sG[(e * 4 + k) * Q3 + q] = F[e][k];
+        }
+    }
+    __syncthreads();
+    // the face-normal fluxes at the lines' ends, and D_d F_d in place of F_d
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+        for (int it = tid; it < 4 * NF; it += NT) {
+            const int k = it / NF, line = it - k * NF;
+            int st;
+            const int base = gl_line_base<NQ>(d, line, st);
+            double* fp = sG + (d * 4 + k) * Q3 + base;
+            double v[NQ], e0, e1;
+#pragma unroll
+            for (int l = 0; l < NQ; ++l) v[l] = fp[l * st];
+            if constexpr (SPLIT) {
+                gl_line_ends<NQ>(T, sR + (d * 4 + k) * Q3 + base, st, e0, e1);
+            } else {
+                e0 = e1 = 0.0;
+#pragma unroll
+                for (int l = 0; l < NQ; ++l) { e0 += T.phis[0][l] * v[l]; e1 += T.phis[1][l] * v[l]; }
+            }
+            tout[((2 * d) * GL_T2W + 4 + k) * NF + line] = -e0;
+            tout[((2 * d + 1) * GL_T2W + 4 + k) * NF + line] = e1;
+#pragma unroll
+            for (int o = 0; o < NQ; ++o) {
+                double x = 0.0;
+#pragma unroll
+                for (int l = 0; l < NQ; ++l) x += T.dphi[o * NQ + l] * v[l];
+                fp[o * st] = x;
+            }
+        }
+    __syncthreads();
+    for (int q = tid; q < Q3; q += NT) {   // W sum_d D_d F_d, momentum and energy rows
+        const double W = wq[q % NQ] * wq[(q / NQ) % NQ] * wq[q / NF];
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            g.vis[((size_t)cell * 4 + k) * Q3 + q] =
+                W * ((sG[k * Q3 + q] + sG[(4 + k) * Q3 + q]) + sG[(8 + k) * Q3 + q]);
+    }
+}
+
 // ------------------------------------------------------------------------------------
 // Residual (+ mass inverse + RK epilogue)
 // ------------------------------------------------------------------------------------
@@ -831,6 +910,37 @@ struct GlStageLayout {
     static constexpr size_t bytes = (size_t)total * sizeof(double);
     static_assert(2 * nT >= 2 * NF * NQ * 5, "the hybrid pair fluxes of one direction fit the temporaries");
 };
+
+// The volume terms at the flux nodes minus the face arrays' lift (see gl_line_ends), plus the viscous
+// divergence. Ends with a barrier.
+template <int NT, int NQ, bool VISC>
+__device__ __forceinline__ void gl_add_faces(const GlTab& T, const GlArgs& g, int cell, const double* sF,
+                                             double* sDiv) {
+    constexpr int NF = NQ * NQ, Q3 = NF * NQ;
+    __shared__ double ph[2][NQ];   // (read with run-time indices)
+    if (threadIdx.x < 2 * NQ) ph[threadIdx.x / NQ][threadIdx.x % NQ] = g.tab->phis[threadIdx.x / NQ][threadIdx.x % NQ];
+    __syncthreads();
+    for (int q = threadIdx.x; q < Q3; q += NT) {
+        const int c[3] = {q % NQ, (q / NQ) % NQ, q / NF};
+        double r[5];
+#pragma unroll
+        for (int s = 0; s < 5; ++s) r[s] = sDiv[s * Q3 + q];
+        if constexpr (VISC) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) r[1 + k] += __ldg(&g.vis[((size_t)cell * 4 + k) * Q3 + q]);
+        }
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            const double p0 = ph[0][c[d]], p1 = ph[1][c[d]];
+            const double* f = sF + 2 * d * 5 * NF + c[d == 2 ? 1 : 2] * NQ + c[d == 0 ? 1 : 0];
+#pragma unroll
+            for (int s = 0; s < 5; ++s) r[s] -= p0 * f[s * NF] + p1 * f[(5 + s) * NF];
+        }
+#pragma unroll
+        for (int s = 0; s < 5; ++s) sDiv[s * Q3 + q] = r[s];
+    }
+    __syncthreads();
+}
 
 // Butcher RK stage (as the collocated kernel's epilogue) of one cell from its time derivative sK
 template <int NT, int D3>
@@ -1197,15 +1307,11 @@ gl_stage_kernel(const StageArgs a, const GlArgs g, const __grid_constant__ GlTab
             __syncthreads();
         }
     }
-    // ---- assembly: r = -chi^T (x3) [div (+ hybrid) + viscous divergence] + sum_f lift(face array), or, on
-    // affine cells, k = M^-1 R straight away: (1/h) (M+K)^-1 (x3) folded into the same passes' operators
-    if constexpr (VISC) {
-        for (int i = threadIdx.x; i < 4 * Q3; i += NT) sDiv[Q3 + i] += __ldg(&g.vis[(size_t)cell * 4 * Q3 + i]);
-        __syncthreads();
-    }
+    // ---- assembly: r = -chi^T (x3) [div (+ hybrid) + viscous divergence - sum_f phis[side] (x) face array],
+    // or, on affine cells, k = M^-1 R straight away: (1/h) (M+K)^-1 (x3) folded into the same passes
+    gl_add_faces<NT, NQ, VISC>(T, g, cell, sF, sDiv);
     if (CURV || a.mode == 0) {
         gl_apply3<NT, ND, NQ, 5, true>(T.chi, sDiv, Q3, sU, D3, t0, t1, -1.0, false);
-        gl_lift_faces<NT, NQ, ND, 5>(sF, 5 * NF, NF, tab->chis[0], tab->chis[1], T.chi, t0, t1, sU, D3, 1.0);
         // affine: sU = R / h^2 (the affine metric C = h^2 I and J = h^2 factored out); curvilinear: R
         if (a.mode == 0) {
             const double h2 = CURV ? 1.0 : a.h * a.h;
@@ -1223,7 +1329,6 @@ gl_stage_kernel(const StageArgs a, const GlArgs g, const __grid_constant__ GlTab
         gl_apply3<NT, ND, NQ, 5>(T.pwa, sDiv, Q3, sQ, D3, t0, t1, 1.0, false);
     } else {
         gl_apply3<NT, ND, NQ, 5, true>(T.chm, sDiv, Q3, sQ, D3, t0, t1, -a.inv_h, false);
-        gl_lift_faces<NT, NQ, ND, 5>(sF, 5 * NF, NF, tab->chms[0], tab->chms[1], T.chm, t0, t1, sQ, D3, a.inv_h);
     }
     if (a.mode == 1) {
         for (int i = threadIdx.x; i < 5 * D3; i += NT) a.out[(size_t)cell * 5 * D3 + i] = sQ[i];
@@ -1286,9 +1391,10 @@ gl_stage_kernel(const StageArgs a, const GlArgs g, const __grid_constant__ GlTab
 // nodes' sums and hands the face sums to the line's first lane, so no pair flux passes through
 // memory. The numerical face fluxes, whose operands come from the face-value buffers, are evaluated
 // while the node quantities are formed. The temporaries of the final passes reuse the space of the
-// quantities (48 KB at NQ = 6: four CTAs per SM). At 12^3 cells of p = 5 it takes 97 us
-// (FP64 pipe 34 % busy, the rest latency); with it, the states projected once and the inverse mass folded
-// into the last passes, a three-stage step of 24^3 such cells takes 7.7 ms instead of 11.9.
+// quantities (48 KB at NQ = 6: four CTAs per SM). At 12^3 cells of p = 5 it takes 86 us
+// (FP64 pipe 37 % busy, the rest latency), 97 us while the faces were lifted one after the other after
+// the last interpolation. A three-stage step of 24^3 such cells: 11.9 ms with the node form, 7.7 with
+// this kernel and the states projected once, 5.1 with the line form of the other two kernels.
 template <int ND, int NQ>
 struct GlLineLayout {
     static constexpr int D3 = ND * ND * ND, Q3 = NQ * NQ * NQ, NF = NQ * NQ;
@@ -1499,19 +1605,14 @@ gl_line_stage_kernel(const StageArgs a, const GlArgs g, const __grid_constant__ 
     }
     __syncthreads();
     // ---- assembly (as gl_stage_kernel's)
-    if constexpr (VISC) {
-        for (int i = tid; i < 4 * Q3; i += NT) sDiv[Q3 + i] += __ldg(&g.vis[(size_t)cell * 4 * Q3 + i]);
-        __syncthreads();
-    }
+    gl_add_faces<NT, NQ, VISC>(T, g, cell, sF, sDiv);
     if (a.mode == 0) {
         gl_apply3<NT, ND, NQ, 5, true>(T.chi, sDiv, Q3, sDiv, D3, t0, t1, -1.0, false);
-        gl_lift_faces<NT, NQ, ND, 5>(sF, 5 * NF, NF, tab->chis[0], tab->chis[1], T.chi, t0, t1, sDiv, D3, 1.0);
         const double h2 = a.h * a.h;
         for (int i = tid; i < 5 * D3; i += NT) a.out[(size_t)cell * 5 * D3 + i] = h2 * sDiv[i];
         return;
     }
     gl_apply3<NT, ND, NQ, 5, true>(T.chm, sDiv, Q3, sDiv, D3, t0, t1, -a.inv_h, false);
-    gl_lift_faces<NT, NQ, ND, 5>(sF, 5 * NF, NF, tab->chms[0], tab->chms[1], T.chm, t0, t1, sDiv, D3, a.inv_h);
     if (a.mode == 1) {
         for (int i = tid; i < 5 * D3; i += NT) a.out[(size_t)cell * 5 * D3 + i] = sDiv[i];
         return;

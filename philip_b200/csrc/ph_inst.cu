@@ -368,10 +368,10 @@ static cudaError_t launch_gl_nq(int kernel, const StageArgs& a, const GlArgs& g,
     constexpr int NT = gl_threads<NQ>();
     static bool cfg[29][64] = {};
     if (kernel == 0) {
-        if (split) return launch_gl_kernel(gl_trace_kernel<ND, NQ, true>, GlTraceLayout<ND, NQ, true>::bytes, NT, a, g, ht,
-                                           cfg[0][dev], s);
-        return launch_gl_kernel(gl_trace_kernel<ND, NQ, false>, GlTraceLayout<ND, NQ, false>::bytes, NT, a, g, ht,
-                                cfg[1][dev], s);
+        if (split) return launch_gl_kernel(gl_trace_kernel<ND, NQ, true>, GlTraceLayout<ND, NQ, true>::bytes,
+                                           GlTraceLayout<ND, NQ, true>::NT, a, g, ht, cfg[0][dev], s);
+        return launch_gl_kernel(gl_trace_kernel<ND, NQ, false>, GlTraceLayout<ND, NQ, false>::bytes,
+                                GlTraceLayout<ND, NQ, false>::NT, a, g, ht, cfg[1][dev], s);
     }
     if (kernel == 1) {
         if (g.vmet && a.btype) {   // curvilinear cells with a boundary face
@@ -392,10 +392,10 @@ static cudaError_t launch_gl_nq(int kernel, const StageArgs& a, const GlArgs& g,
             return launch_gl_kernel(gl_aux_kernel<ND, NQ, false, false, true>, GlAuxLayout<ND, NQ, false>::bytes, NT, a,
                                     g, ht, cfg[16][dev], s);
         }
-        if (split) return launch_gl_kernel(gl_aux_kernel<ND, NQ, true>, GlAuxLayout<ND, NQ, true>::bytes, NT, a, g, ht,
-                                           cfg[2][dev], s);
-        return launch_gl_kernel(gl_aux_kernel<ND, NQ, false>, GlAuxLayout<ND, NQ, false>::bytes, NT, a, g, ht,
-                                cfg[3][dev], s);
+        if (split) return launch_gl_kernel(gl_aux_line_kernel<ND, NQ, true>, GlAuxLineLayout<ND, NQ, true>::bytes,
+                                           GlAuxLineLayout<ND, NQ, true>::NT, a, g, ht, cfg[2][dev], s);
+        return launch_gl_kernel(gl_aux_line_kernel<ND, NQ, false>, GlAuxLineLayout<ND, NQ, false>::bytes,
+                                GlAuxLineLayout<ND, NQ, false>::NT, a, g, ht, cfg[3][dev], s);
     }
     if (kernel == 3)   // curvilinear: the weight-adjusted inverse mass alone
         return launch_gl_kernel(gl_minv_kernel<ND, NQ>, GlMinvLayout<ND, NQ>::bytes, NT, a, g, ht, cfg[8][dev], s);
