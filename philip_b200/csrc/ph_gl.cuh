@@ -361,7 +361,8 @@ __device__ __forceinline__ void gl_load_tab(const GlTab* g, GlTab* s, int nt) {
 // ------------------------------------------------------------------------------------
 template <int ND, int NQ, bool SPLIT>
 struct GlTraceLayout {
-    static constexpr int NT = NQ == 6 ? 192 : gl_threads<NQ>();     // 180 lines per pass at NQ = 6
+    // the lines of five rows in one pass (80 at NQ = 4, 180 at NQ = 6)
+    static constexpr int NT = NQ == 4 ? 96 : NQ == 6 ? 192 : gl_threads<NQ>();
     static constexpr int D3 = ND * ND * ND, Q3 = NQ * NQ * NQ;
     static constexpr int oQ = 0;                                    // 5 NQ^3 (flux-node values / entropy variables)
     static constexpr int nW = 5 * Q3;
@@ -728,7 +729,7 @@ gl_aux_kernel(const StageArgs a, const GlArgs g, const __grid_constant__ GlTab T
 // direction's five rows in one pass.
 template <int ND, int NQ, bool SPLIT>
 struct GlAuxLineLayout {
-    static constexpr int NT = NQ <= 4 ? 64 : NQ == 5 ? 128 : NQ == 6 ? 192 : 256;
+    static constexpr int NT = NQ <= 3 ? 64 : NQ == 4 ? 96 : NQ == 5 ? 128 : NQ == 6 ? 192 : 256;
     static constexpr int D3 = ND * ND * ND, Q3 = NQ * NQ * NQ, NF = NQ * NQ;
     static constexpr int oQ = 0;                          // 5 NQ^3 state at the flux nodes
     static constexpr int oG = oQ + 5 * Q3;                // 15 NQ^3 lifted gradient, later flux rows d * 4 + k
@@ -737,7 +738,7 @@ struct GlAuxLineLayout {
     static constexpr int total = oR + nR;
     static constexpr size_t bytes = (size_t)total * sizeof(double);
     // CTAs per SM asked of the register allocator (96 registers at NQ = 6)
-    static constexpr int MINB = NQ <= 4 ? 8 : NQ == 5 ? 4 : NQ == 6 ? 3 : 2;
+    static constexpr int MINB = NQ <= 3 ? 8 : NQ == 4 ? 5 : NQ == 5 ? 4 : NQ == 6 ? 3 : 2;
 };
 
 template <int ND, int NQ, bool SPLIT>
@@ -1381,6 +1382,172 @@ gl_stage_kernel(const StageArgs a, const GlArgs g, const __grid_constant__ GlTab
     gl_rk_epilogue<NT, D3>(a, cell, sQ);
 }
 
+// The last part of the affine stage kernels (as gl_stage_kernel's): lifts, transposed interpolation with the
+// inverse mass, and the result or the RK stage. Overwrites sDiv.
+template <int NT, int ND, int NQ, bool VISC>
+__device__ __forceinline__ void gl_finish(const StageArgs& a, const GlTab& T, const GlArgs& g, int cell,
+                                          const double* sF, double* sDiv, double* t0, double* t1) {
+    constexpr int D3 = ND * ND * ND, Q3 = NQ * NQ * NQ;
+    gl_add_faces<NT, NQ, VISC>(T, g, cell, sF, sDiv);
+    if (a.mode == 0) {
+        gl_apply3<NT, ND, NQ, 5, true>(T.chi, sDiv, Q3, sDiv, D3, t0, t1, -1.0, false);
+        const double h2 = a.h * a.h;
+        for (int i = threadIdx.x; i < 5 * D3; i += NT) a.out[(size_t)cell * 5 * D3 + i] = h2 * sDiv[i];
+        return;
+    }
+    gl_apply3<NT, ND, NQ, 5, true>(T.chm, sDiv, Q3, sDiv, D3, t0, t1, -a.inv_h, false);
+    if (a.mode == 1) {
+        for (int i = threadIdx.x; i < 5 * D3; i += NT) a.out[(size_t)cell * 5 * D3 + i] = sDiv[i];
+        return;
+    }
+    if (a.mode == 3) {   // low-storage 3S* / 3S*+ stage
+        double err2 = 0.0;
+        for (int i = threadIdx.x; i < 5 * D3; i += NT) ls_stage_dof(a, (size_t)cell * 5 * D3 + i, sDiv[i], err2);
+        if (a.err_partial) ls_tile_error<NT>(err2, &a.err_partial[cell]);
+        return;
+    }
+    gl_rk_epilogue<NT, D3>(a, cell, sDiv);
+}
+
+// ------------------------------------------------------------------------------------
+// Residual (+ mass inverse + RK epilogue), conservative form, affine cells without boundary faces
+// ------------------------------------------------------------------------------------
+// One CTA per cell with a thread per line of one direction's five rows. A direction's flux lines give
+// the volume flux at their ends and are replaced by their derivatives in one pass, the numerical fluxes
+// are evaluated in the face's frame (the normal's axis first, so that the penalty's jump has one
+// direction), and the state, the fluxes and the temporaries share their space (14 KB at NQ = 4). Bound by
+// latency: a step of 12^3 cells of p = 3 (Roe, SIPG, three stages) takes 160 us where gl_stage_kernel with two
+// warps of 236 registers a cell took 228.
+template <int ND, int NQ>
+struct GlConsLayout {
+    static constexpr int NT = NQ <= 3 ? 64 : NQ == 4 ? 96 : NQ == 5 ? 160 : NQ == 6 ? 224 : 256;
+    static constexpr int MINB = 512 / NT;                 // 128 registers
+    static constexpr int D3 = ND * ND * ND, Q3 = NQ * NQ * NQ, NF = NQ * NQ;
+    static constexpr int oQ = 0;                          // 5 NQ^3 state at the flux nodes, later the volume terms
+    static constexpr int oN = oQ + 5 * Q3;                // [d][s][Q3] fluxes, then derivatives; temporaries
+    static constexpr int oF = oN + 15 * Q3;               // [face][5][NF] face arrays
+    static constexpr int total = oF + 30 * NF;
+    static constexpr size_t bytes = (size_t)total * sizeof(double);
+};
+
+template <int ND, int NQ, bool VISC>
+__global__ void __launch_bounds__(GlConsLayout<ND, NQ>::NT, GlConsLayout<ND, NQ>::MINB)
+gl_cons_stage_kernel(const StageArgs a, const GlArgs g, const __grid_constant__ GlTab T) {
+    using L = GlConsLayout<ND, NQ>;
+    constexpr int NT = L::NT, D3 = L::D3, Q3 = L::Q3, NF = L::NF, T1W = gl_t1_width<false>();
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ double wq[NQ];
+    double* sm = reinterpret_cast<double*>(smem_raw);
+    double* sQ = sm + L::oQ;
+    double* sN = sm + L::oN;
+    double* sF = sm + L::oF;
+    double* t0 = sN;
+    double* t1 = sN + 5 * Q3;
+    const int cell = a.tiles ? __ldg(&a.tiles[blockIdx.x]) : a.cell_begin + (int)blockIdx.x;
+    const int tid = threadIdx.x;
+    Cst<double> cst; cst.load(a.pc);
+    const int tp = a.pc.two_point, cf = a.pc.conv_flux, df = a.pc.diss_flux, ucv = a.pc.use_const_visc;
+    if (tid < NQ) wq[tid] = g.tab->wq[tid];
+    for (int i = tid; i < 5 * D3; i += NT) sQ[i] = __ldg(&a.U[(size_t)cell * 5 * D3 + i]);
+    gl_prefetch_l2<NT, NF, D3, Q3, T1W, true, VISC>(a, g, cell);
+    __syncthreads();
+    gl_apply3<NT, NQ, ND, 5>(T.chi, sQ, D3, sQ, Q3, t0, t1, 1.0, false);
+    for (int q = tid; q < Q3; q += NT) {
+        double u[5];
+#pragma unroll
+        for (int s = 0; s < 5; ++s) u[s] = sQ[s * Q3 + q];
+        NodeQ<double> nq;
+        node_prepare<double>(u, TP_KG, cst.gm1, nq, a.status);
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            const double nv[3] = {d == 0 ? 1.0 : 0.0, d == 1 ? 1.0 : 0.0, d == 2 ? 1.0 : 0.0};
+            double F[5];
+            conv_flux_n<double>(nq, nv, 0.0, F);
+#pragma unroll
+            for (int s = 0; s < 5; ++s) sN[(d * 5 + s) * Q3 + q] = F[s];
+        }
+    }
+    __syncthreads();
+    // D_d F_d in place of F_d, and the cell's own flux n . F at the lines' ends   (strong_dg.cpp:1546)
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+        for (int it = tid; it < 5 * NF; it += NT) {
+            const int s = it / NF, line = it - s * NF;
+            int st;
+            double* fp = sN + (d * 5 + s) * Q3 + gl_line_base<NQ>(d, line, st);
+            double v[NQ], e0 = 0.0, e1 = 0.0;
+#pragma unroll
+            for (int l = 0; l < NQ; ++l) v[l] = fp[l * st];
+#pragma unroll
+            for (int l = 0; l < NQ; ++l) { e0 += T.phis[0][l] * v[l]; e1 += T.phis[1][l] * v[l]; }
+            sF[(2 * d * 5 + s) * NF + line] = -e0;
+            sF[((2 * d + 1) * 5 + s) * NF + line] = e1;
+#pragma unroll
+            for (int o = 0; o < NQ; ++o) {
+                double x = 0.0;
+#pragma unroll
+                for (int l = 0; l < NQ; ++l) x += T.dphi[o * NQ + l] * v[l];
+                fp[o * st] = x;
+            }
+        }
+    __syncthreads();
+    for (int q = tid; q < Q3; q += NT) {
+        const double W = wq[q % NQ] * wq[(q / NQ) % NQ] * wq[q / NF];
+#pragma unroll
+        for (int s = 0; s < 5; ++s)
+            sQ[s * Q3 + q] = W * ((sN[s * Q3 + q] + sN[(5 + s) * Q3 + q]) + sN[(10 + s) * Q3 + q]);
+    }
+    // numerical fluxes (canonical orientation: the left state is the cell whose +e_d face it is)
+#pragma unroll 1
+    for (int it = tid; it < 6 * NF; it += NT) {
+        const int f = it / NF, q2 = it - f * NF;
+        const int d = f >> 1, side = f & 1;
+        const int d2 = d == 2 ? 0 : d + 1, d3 = d == 0 ? 2 : d - 1;
+        const double sgn = side ? 1.0 : -1.0;
+        const int cn = __ldg(&a.nbr[cell * 6 + f]);
+        const double* to = g.t1 + ((size_t)cell * 6 + f) * T1W * NF + q2;
+        const double* te = g.t1 + ((size_t)cn * 6 + (f ^ 1)) * T1W * NF + q2;
+        const int row[5] = {0, 1 + d, 1 + d2, 1 + d3, 4};
+        double uL[5], uR[5], term[5];
+#pragma unroll
+        for (int s = 0; s < 5; ++s) {
+            const double uo = __ldg(&to[row[s] * NF]), ue = __ldg(&te[row[s] * NF]);
+            uL[s] = side ? uo : ue;
+            uR[s] = side ? ue : uo;
+        }
+        NodeQ<double> qL, qR;
+        node_prepare<double>(uL, tp, cst.gm1, qL, nullptr);
+        node_prepare<double>(uR, tp, cst.gm1, qR, nullptr);
+        conv_num_flux<double, 0>(uL, uR, qL, qR, tp, cf, cst, term);
+        if constexpr (VISC) {   // each side's F_v(u, q) . e_d at the face node, from the auxiliary kernel
+            const double* ao = g.t2 + ((size_t)cell * 6 + f) * GL_T2W * NF + q2;
+            const double* ae = g.t2 + ((size_t)cn * 6 + (f ^ 1)) * GL_T2W * NF + q2;
+            const int kr[4] = {d, d2, d3, 3};
+            double Fd[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) Fd[k] = 0.5 * (__ldg(&ao[kr[k] * NF]) + __ldg(&ae[kr[k] * NF]));
+            if (df == DF_SIPG) {
+                double jump[5][3], AL[3][4], AR[3][4];
+#pragma unroll
+                for (int s = 0; s < 5; ++s) { jump[s][0] = uL[s] - uR[s]; jump[s][1] = jump[s][2] = 0.0; }
+                viscous_flux<double>(uL, jump, ucv, cst, AL, 1, nullptr);
+                viscous_flux<double>(uR, jump, ucv, cst, AR, 1, nullptr);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) Fd[k] -= a.pen * (0.5 * (AL[0][k] + AR[0][k]));
+            }
+#pragma unroll
+            for (int k = 0; k < 4; ++k) term[1 + k] += Fd[k] - sgn * __ldg(&ao[(4 + kr[k]) * NF]);
+        }
+        const double wf = wq[q2 % NQ] * wq[q2 / NQ];
+#pragma unroll
+        for (int s = 0; s < 5; ++s) {
+            double* o = sF + (f * 5 + row[s]) * NF + q2;
+            *o = wf * (*o - sgn * term[s]);
+        }
+    }
+    gl_finish<NT, ND, NQ, VISC>(a, T, g, cell, sF, sQ, t0, t1);
+}
+
 // ------------------------------------------------------------------------------------
 // Residual (+ mass inverse + RK epilogue), Chandrashekar + EC/Roe (+ BR2) flux set, affine cells
 // without boundary faces
@@ -1604,26 +1771,7 @@ gl_line_stage_kernel(const StageArgs a, const GlArgs g, const __grid_constant__ 
         }
     }
     __syncthreads();
-    // ---- assembly (as gl_stage_kernel's)
-    gl_add_faces<NT, NQ, VISC>(T, g, cell, sF, sDiv);
-    if (a.mode == 0) {
-        gl_apply3<NT, ND, NQ, 5, true>(T.chi, sDiv, Q3, sDiv, D3, t0, t1, -1.0, false);
-        const double h2 = a.h * a.h;
-        for (int i = tid; i < 5 * D3; i += NT) a.out[(size_t)cell * 5 * D3 + i] = h2 * sDiv[i];
-        return;
-    }
-    gl_apply3<NT, ND, NQ, 5, true>(T.chm, sDiv, Q3, sDiv, D3, t0, t1, -a.inv_h, false);
-    if (a.mode == 1) {
-        for (int i = tid; i < 5 * D3; i += NT) a.out[(size_t)cell * 5 * D3 + i] = sDiv[i];
-        return;
-    }
-    if (a.mode == 3) {   // low-storage 3S* / 3S*+ stage
-        double err2 = 0.0;
-        for (int i = tid; i < 5 * D3; i += NT) ls_stage_dof(a, (size_t)cell * 5 * D3 + i, sDiv[i], err2);
-        if (a.err_partial) ls_tile_error<NT>(err2, &a.err_partial[cell]);
-        return;
-    }
-    gl_rk_epilogue<NT, D3>(a, cell, sDiv);
+    gl_finish<NT, ND, NQ, VISC>(a, T, g, cell, sF, sDiv, t0, t1);
 }
 
 // ------------------------------------------------------------------------------------
