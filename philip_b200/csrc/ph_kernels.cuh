@@ -1123,19 +1123,17 @@ residual_kernel_batched(const StageArgs* __restrict__ inst, const BatchTile* __r
 // needs: its volume divergence and its face-normal component on each face
 // (viscous_terms_per_cell).
 // ------------------------------------------------------------------------------------
-// Two forms of the same arithmetic, chosen per order from timings on B200:
-//  line form (p >= 4): one thread per (direction, state, line) differentiates the line held
-//    in registers; every coefficient is a parameter-bank operand, the gradient and then the
-//    nodal flux share one buffer, the divergence runs direction by direction (at p = 5 it
-//    takes 0.170 ms against 0.262 ms for the node form in FP64, 0.124 against 0.162 in FP32);
-//  node form (p <= 3): one thread per node, coefficients from shared memory (fewer barriers
-//    and less shared memory, which wins at low order).
-// Both sum every node's terms in the same order (over l, then over directions).
+// One thread per (direction, state, line) differentiates the line held in registers: every
+// coefficient is a parameter-bank operand, the gradient and then the nodal flux share one buffer, and
+// in FP64 every direction's derivative takes its flux's place and the three are summed as they are stored
+// (FP32 adds direction by direction into the state's rows, so that its rounding stays what it is).
+// Bound by shared memory (84 % of its wavefronts at p = 5): lines along x move as pairs, which leaves
+// two-way conflicts along y only. Timed on B200 at 24^3 cells, p = 5: 0.140 ms in FP64 (0.148 with scalar
+// x-lines and a divergence summed in shared memory), 0.094 in FP32 (0.099). At p <= 3 a thread per node
+// with the coefficients in shared memory was the other form: 32^3 cells p = 3 0.142 against 0.127 here in
+// FP64 and 0.090 against 0.076 in FP32, p = 2 0.078 / 0.063 and 0.053 / 0.048, p = 1 0.023 / 0.021.
 // An FR auxiliary correction (K_aux != 0) multiplies the gradient by Baux(x)Baux(x)Baux before
-// the flux; it needs the whole gradient in shared memory, so it always takes the line form.
-template <typename R, int N1, bool FRA = false> __host__ __device__ constexpr bool aux_line_form() {
-    return N1 >= 5 || FRA;
-}
+// the flux.
 
 // CTAs per SM of the periodic FP64 auxiliary kernel at p = 5 (224 threads). Timed on B200 at
 // 24^3 cells inside the RK4 steps: 3 (76 registers) 0.163 ms, 4 (70 registers) 0.147 ms, 5 (56
@@ -1149,18 +1147,17 @@ template <int N1, int CPC, bool FRA = false>
 struct AuxLayout {
     static constexpr int NP = N1 * N1 * N1, NF = N1 * N1;
     static constexpr int NT = ((CPC * NP + 31) / 32) * 32 > 512 ? 512 : ((CPC * NP + 31) / 32) * 32;
-    // CTAs per SM asked of the register allocator (the periodic FP64 line form at p = 5 with one
+    // CTAs per SM asked of the register allocator (the periodic FP64 kernel at p = 5 with one
     // cell per CTA; the other forms take what they need)
     template <typename R, bool CURV, bool BND>
     static constexpr int minb() {
         return (sizeof(R) == 8 && N1 == 6 && CPC == 1 && !FRA && !CURV && !BND) ? PH_AUX_P5_MINB : 1;
     }
-    // state, neighbour traces, then (line form) the gradient / nodal flux or (node form) the
-    // differentiation matrix and the nodal flux
+    // state, neighbour traces, then the gradient / nodal flux
     template <typename R>
     static constexpr size_t bytes() {
         return sizeof(R) * ((size_t)CPC * 5 * NP + (size_t)CPC * 6 * 5 * NF +
-                            (aux_line_form<R, N1, FRA>() ? (size_t)CPC * 15 * NP : N1 * N1 + (size_t)CPC * 12 * NP));
+                            (size_t)CPC * 15 * NP);
     }
 };
 
@@ -1330,6 +1327,40 @@ __device__ __forceinline__ void aux_boundary_node(const int* __restrict__ nbr, c
     aux_boundary_fluxes<R, N1>(nbr, btype, Fb, cell, node, uu, gg, pc, pen, metric);
 }
 
+// One line of N1 values at stride ST in shared memory, to and from registers. Lines along x at even N1 are
+// contiguous and move two values at a time: a stride of N1 values between threads puts scalar accesses
+// two to a bank, pairs of them none.
+template <typename R, int N1, int ST> __device__ __forceinline__ void line_load(const R* p, R v[N1]) {
+    using R2 = std::conditional_t<sizeof(R) == 8, double2, float2>;
+    if constexpr (ST == 1 && N1 % 2 == 0) {
+#pragma unroll
+        for (int l = 0; l < N1; l += 2) {
+            const R2 t = *reinterpret_cast<const R2*>(p + l);
+            v[l] = t.x;
+            v[l + 1] = t.y;
+        }
+    } else {
+#pragma unroll
+        for (int l = 0; l < N1; ++l) v[l] = p[l * ST];
+    }
+}
+template <typename R, int N1, int ST> __device__ __forceinline__ void line_store(R* p, const R v[N1]) {
+    using R2 = std::conditional_t<sizeof(R) == 8, double2, float2>;
+    if constexpr (ST == 1 && N1 % 2 == 0) {
+#pragma unroll
+        for (int l = 0; l < N1; l += 2) {
+            R2 t;
+            t.x = v[l];
+            t.y = v[l + 1];
+            *reinterpret_cast<R2*>(p + l) = t;
+        }
+    } else {
+#pragma unroll
+        for (int l = 0; l < N1; ++l) p[l * ST] = v[l];
+    }
+}
+template <int D> struct AuxDir { static constexpr int d = D; };
+
 template <typename R, int N1, int CPC, bool FRA, bool CURV, bool BND = false>
 __global__ void __launch_bounds__(AuxLayout<N1, CPC, FRA>::NT, AuxLayout<N1, CPC, FRA>::template minb<R, CURV, BND>())
 aux_kernel(const double* __restrict__ U, const int* __restrict__ nbr, int cell_begin, int nc, R inv_h, PhysConst pc,
@@ -1377,209 +1408,159 @@ aux_kernel(const double* __restrict__ U, const int* __restrict__ nbr, int cell_b
 #pragma unroll
         for (int s = 0; s < 5; ++s) dst[s * NF] = (R)__ldg(&src[s * NP]);
     }
-    if constexpr (aux_line_form<R, N1, FRA>()) {
-        R* sG = sT + CPC * 6 * 5 * NF;   // [c][d][5][NP] gradient, later [c][d][4][NP] flux
-        __syncthreads();
-        // lifted gradient: D u along the line, the lifting u* - u = (u_ext - u)/2 at both ends;
-        // the direction is a compile-time constant, so the line's stride is too
+    R* sG = sT + CPC * 6 * 5 * NF;   // [c][d][5][NP] gradient, later [c][d][4][NP] flux
+    // FP32 up to p = 3: 1/h is applied as the gradient is read, where it joins the flux's first operation
+    constexpr bool LATE = sizeof(R) == 4 && N1 <= 4 && !FRA;
+    __syncthreads();
+    // lifted gradient: D u along the line, the lifting u* - u = (u_ext - u)/2 at both ends;
+    // the direction is a compile-time constant, so the line's stride is too
+    auto gradient = [&](auto dir) {
+        constexpr int d = decltype(dir)::d, st = d == 0 ? 1 : d == 1 ? N1 : N1 * N1;
+        for (int task = tid; task < CPC * 5 * NF; task += NT) {
+            const int c = task / (5 * NF), r = task % (5 * NF);
+            const int line = r % NF, s = r / NF;
+            const int base = line_node<N1>(d, line, 0);
+            R v[N1], o[N1];
+            line_load<R, N1, st>(sU + (c * 5 + s) * NP + base, v);
+            const R ue0 = sT[((c * 6 + 2 * d) * 5 + s) * NF + line];
+            const R ue1 = sT[((c * 6 + 2 * d + 1) * 5 + s) * NF + line];
 #pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            const int st = d == 0 ? 1 : d == 1 ? N1 : N1 * N1;
-            for (int task = tid; task < CPC * 5 * NF; task += NT) {
-                const int c = task / (5 * NF), r = task % (5 * NF);
-                const int line = r % NF, s = r / NF;
-                const int base = line_node<N1>(d, line, 0);
-                const R* u = sU + (c * 5 + s) * NP + base;
+            for (int pos = 0; pos < N1; ++pos) {
+                R acc = R(0);
+#pragma unroll
+                for (int l = 0; l < N1; ++l) acc += co.D[pos * MAXN1 + l] * v[l];
+                if (pos == 0) acc += co.inv_wend * (-(R(0.5) * (v[0] + ue0) - v[0]));
+                if (pos == N1 - 1) acc += co.inv_wend * ((R(0.5) * (v[N1 - 1] + ue1) - v[N1 - 1]));
+                o[pos] = LATE ? acc : acc * inv_h;
+            }
+            line_store<R, N1, st>(sG + (c * 15 + d * 5 + s) * NP + base, o);
+        }
+    };
+    gradient(AuxDir<0>());
+    gradient(AuxDir<1>());
+    gradient(AuxDir<2>());
+    __syncthreads();
+    if constexpr (FRA) {
+        // FR auxiliary correction (M+K_aux)^{-1} in three directions, applied to the DG
+        // gradient diag(w)^{-1} r as Baux = (M+K_aux)^{-1} diag(w) along x, then y, then z
+        // (the order of the sum-factorised inverse mass); one thread per (component, line)
+#pragma unroll
+        for (int e = 0; e < 3; ++e) {
+            const int st = e == 0 ? 1 : e == 1 ? N1 : N1 * N1;
+            for (int task = tid; task < CPC * 15 * NF; task += NT) {
+                const int c = task / (15 * NF), r = task % (15 * NF);
+                const int line = r % NF, k = r / NF;
+                R* g = sG + (c * 15 + k) * NP + line_node<N1>(e, line, 0);
                 R v[N1];
 #pragma unroll
-                for (int l = 0; l < N1; ++l) v[l] = u[l * st];
-                const R ue0 = sT[((c * 6 + 2 * d) * 5 + s) * NF + line];
-                const R ue1 = sT[((c * 6 + 2 * d + 1) * 5 + s) * NF + line];
-                R* g = sG + (c * 15 + d * 5 + s) * NP + base;
+                for (int l = 0; l < N1; ++l) v[l] = g[l * st];
 #pragma unroll
                 for (int pos = 0; pos < N1; ++pos) {
                     R acc = R(0);
 #pragma unroll
-                    for (int l = 0; l < N1; ++l) acc += co.D[pos * MAXN1 + l] * v[l];
-                    if (pos == 0) acc += co.inv_wend * (-(R(0.5) * (v[0] + ue0) - v[0]));
-                    if (pos == N1 - 1) acc += co.inv_wend * ((R(0.5) * (v[N1 - 1] + ue1) - v[N1 - 1]));
-                    g[pos * st] = acc * inv_h;
+                    for (int l = 0; l < N1; ++l) acc += co.Ba[pos * MAXN1 + l] * v[l];
+                    g[pos * st] = acc;
                 }
             }
+            __syncthreads();
         }
+    }
+    // viscous flux per node; it replaces the node's own gradient entries
+    for (int it = tid; it < CPC * NP; it += NT) {
+        const int c = it / NP, node = it % NP;
+        R g[5][3];
+#pragma unroll
+        for (int d = 0; d < 3; ++d)
+#pragma unroll
+            for (int s = 0; s < 5; ++s)
+                g[s][d] = LATE ? sG[(c * 15 + d * 5 + s) * NP + node] * inv_h : sG[(c * 15 + d * 5 + s) * NP + node];
+        R un[5];
+#pragma unroll
+        for (int s = 0; s < 5; ++s) un[s] = sU[(c * 5 + s) * NP + node];
+        R F[3][4];
+        if constexpr (CURV) {
+            int cell = cell0 + c; if (cell >= nc) cell = nc - 1;
+            aux_curv_flux<R, N1>(un, g, metric, cell, node, pc.use_const_visc, cst, F);
+        } else {
+            viscous_flux<R>(un, g, pc.use_const_visc, cst, F, 7, nullptr);
+        }
+        if constexpr (BND) {
+            if (cell0 + c < nc)
+                aux_boundary_node<R, N1>(nbr, btype, Fb, cell0 + c, node, un, g, pc, pen, CURV ? metric : nullptr);
+        }
+#pragma unroll
+        for (int d = 0; d < 3; ++d)
+#pragma unroll
+            for (int k = 0; k < 4; ++k) sG[(c * 15 + d * 4 + k) * NP + node] = F[d][k];
+    }
+    // divergence sum_d D_d F_d, one thread per (component, line), which also stores the line's face values
+    auto derivative = [&](auto dir, int c, int k, int line, R o[N1]) {
+        constexpr int d = decltype(dir)::d, st = d == 0 ? 1 : d == 1 ? N1 : N1 * N1;
+        R v[N1];
+        line_load<R, N1, st>(sG + (c * 15 + d * 4 + k) * NP + line_node<N1>(d, line, 0), v);
+#pragma unroll
+        for (int pos = 0; pos < N1; ++pos)
+#pragma unroll
+            for (int l = 0; l < N1; ++l) o[pos] += co.D[pos * MAXN1 + l] * v[l];
+        if (cell0 + c < nc) {
+            R* dst = Fv + (size_t)(cell0 + c) * VT + 4 * NP + (2 * d * 4 + k) * NF + line;
+            dst[0] = v[0];
+            dst[4 * NF] = v[N1 - 1];
+        }
+    };
+    if constexpr (sizeof(R) == 8) {
+        // FP64: every direction's derivative in place of its flux, summed as it is stored
+        auto inplace = [&](auto dir) {
+            constexpr int d = decltype(dir)::d, st = d == 0 ? 1 : d == 1 ? N1 : N1 * N1;
+            for (int task = tid; task < CPC * 4 * NF; task += NT) {
+                const int c = task / (4 * NF), r = task % (4 * NF);
+                const int line = r % NF, k = r / NF;
+                R o[N1];
+#pragma unroll
+                for (int pos = 0; pos < N1; ++pos) o[pos] = R(0);
+                derivative(dir, c, k, line, o);
+                line_store<R, N1, st>(sG + (c * 15 + d * 4 + k) * NP + line_node<N1>(d, line, 0), o);
+            }
+        };
         __syncthreads();
-        if constexpr (FRA) {
-            // FR auxiliary correction (M+K_aux)^{-1} in three directions, applied to the DG
-            // gradient diag(w)^{-1} r as Baux = (M+K_aux)^{-1} diag(w) along x, then y, then z
-            // (the order of the sum-factorised inverse mass); one thread per (component, line)
-#pragma unroll
-            for (int e = 0; e < 3; ++e) {
-                const int st = e == 0 ? 1 : e == 1 ? N1 : N1 * N1;
-                for (int task = tid; task < CPC * 15 * NF; task += NT) {
-                    const int c = task / (15 * NF), r = task % (15 * NF);
-                    const int line = r % NF, k = r / NF;
-                    R* g = sG + (c * 15 + k) * NP + line_node<N1>(e, line, 0);
-                    R v[N1];
-#pragma unroll
-                    for (int l = 0; l < N1; ++l) v[l] = g[l * st];
-#pragma unroll
-                    for (int pos = 0; pos < N1; ++pos) {
-                        R acc = R(0);
-#pragma unroll
-                        for (int l = 0; l < N1; ++l) acc += co.Ba[pos * MAXN1 + l] * v[l];
-                        g[pos * st] = acc;
-                    }
-                }
-                __syncthreads();
-            }
+        inplace(AuxDir<0>());
+        inplace(AuxDir<1>());
+        inplace(AuxDir<2>());
+        __syncthreads();
+        for (int it = tid; it < CPC * 4 * NP; it += NT) {
+            const int c = it / (4 * NP), i = it % (4 * NP);
+            const R* f = sG + c * 15 * NP + i;
+            if (cell0 + c < nc) Fv[(size_t)(cell0 + c) * VT + i] = (f[0] + f[4 * NP]) + f[8 * NP];
         }
-        // viscous flux per node; it replaces the node's own gradient entries
-        for (int it = tid; it < CPC * NP; it += NT) {
-            const int c = it / NP, node = it % NP;
-            R g[5][3];
-#pragma unroll
-            for (int d = 0; d < 3; ++d)
-#pragma unroll
-                for (int s = 0; s < 5; ++s) g[s][d] = sG[(c * 15 + d * 5 + s) * NP + node];
-            R un[5];
-#pragma unroll
-            for (int s = 0; s < 5; ++s) un[s] = sU[(c * 5 + s) * NP + node];
-            R F[3][4];
-            if constexpr (CURV) {
-                int cell = cell0 + c; if (cell >= nc) cell = nc - 1;
-                aux_curv_flux<R, N1>(un, g, metric, cell, node, pc.use_const_visc, cst, F);
-            } else {
-                viscous_flux<R>(un, g, pc.use_const_visc, cst, F, 7, nullptr);
-            }
-            if constexpr (BND) {
-                if (cell0 + c < nc)
-                    aux_boundary_node<R, N1>(nbr, btype, Fb, cell0 + c, node, un, g, pc, pen, CURV ? metric : nullptr);
-            }
-#pragma unroll
-            for (int d = 0; d < 3; ++d)
-#pragma unroll
-                for (int k = 0; k < 4; ++k) sG[(c * 15 + d * 4 + k) * NP + node] = F[d][k];
-        }
-        // divergence sum_d D_d F_d into the state's rows (the state is no longer read), one
-        // direction after the other, one thread per (component, line)
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            const int st = d == 0 ? 1 : d == 1 ? N1 : N1 * N1;
+    } else {
+        // FP32: into the state's rows (the state is no longer read), one direction after the other
+        auto summed = [&](auto dir) {
+            constexpr int d = decltype(dir)::d, st = d == 0 ? 1 : d == 1 ? N1 : N1 * N1;
             __syncthreads();
             for (int task = tid; task < CPC * 4 * NF; task += NT) {
                 const int c = task / (4 * NF), r = task % (4 * NF);
                 const int line = r % NF, k = r / NF;
-                const int base = line_node<N1>(d, line, 0);
-                const R* f = sG + (c * 15 + d * 4 + k) * NP + base;
-                R* dv = sU + (c * 4 + k) * NP + base;
-                R v[N1];
+                R* dv = sU + (c * 4 + k) * NP + line_node<N1>(d, line, 0);
+                R o[N1];
+                if constexpr (d == 0) {
 #pragma unroll
-                for (int l = 0; l < N1; ++l) v[l] = f[l * st];
-#pragma unroll
-                for (int pos = 0; pos < N1; ++pos) {
-                    R acc = d == 0 ? R(0) : dv[pos * st];
-#pragma unroll
-                    for (int l = 0; l < N1; ++l) acc += co.D[pos * MAXN1 + l] * v[l];
-                    dv[pos * st] = acc;
+                    for (int pos = 0; pos < N1; ++pos) o[pos] = R(0);
+                } else {
+                    line_load<R, N1, st>(dv, o);
                 }
+                derivative(dir, c, k, line, o);
+                line_store<R, N1, st>(dv, o);
             }
-        }
+        };
+        summed(AuxDir<0>());
+        summed(AuxDir<1>());
+        summed(AuxDir<2>());
         __syncthreads();
         for (int it = tid; it < CPC * 4 * NP; it += NT) {
             const int c = it / (4 * NP);
             const int cell = cell0 + c;
             if (cell >= nc) continue;
             Fv[(size_t)cell * VT + it % (4 * NP)] = sU[c * 4 * NP + it % (4 * NP)];
-        }
-        for (int it = tid; it < CPC * 6 * NF; it += NT) {   // one thread per (cell, face, face node)
-            const int c = it / (6 * NF), j = it % (6 * NF);
-            const int cell = cell0 + c;
-            if (cell >= nc) continue;
-            const int f = j / NF, fn = j % NF;
-            const int d = f >> 1;
-            const int node = line_node<N1>(d, fn, (f & 1) ? N1 - 1 : 0);
-            R* dst = Fv + (size_t)cell * VT + 4 * NP + f * 4 * NF + fn;
-            const R* src = sG + (c * 15 + d * 4) * NP + node;
-#pragma unroll
-            for (int k = 0; k < 4; ++k) dst[k * NF] = src[k * NP];
-        }
-    } else {
-        R* sDm = sT + CPC * 6 * 5 * NF;
-        R* sF = sDm + N1 * N1;   // [c][3 dirs x 4][NP] nodal viscous flux
-        for (int i = tid; i < N1 * N1; i += NT) sDm[i] = co.D[(i / N1) * MAXN1 + (i % N1)];
-        __syncthreads();
-        for (int it = tid; it < CPC * NP; it += NT) {
-            const int c = it / NP, node = it % NP;
-            const int cell = cell0 + c;
-            if (cell >= nc) continue;
-            const int cx[3] = {node % N1, (node / N1) % N1, node / (N1 * N1)};
-            const R* u = sU + c * 5 * NP;
-            R g[5][3];
-#pragma unroll
-            for (int d = 0; d < 3; ++d) {
-                const int st = (d == 0) ? 1 : (d == 1) ? N1 : N1 * N1;
-                const int pos = cx[d];
-                const int base = node - pos * st;
-                const int t1 = (d == 0) ? 1 : 0, t2 = (d == 2) ? 1 : 2;
-                const int fn = cx[t2] * N1 + cx[t1];
-#pragma unroll
-                for (int s = 0; s < 5; ++s) {
-                    R v = R(0);
-#pragma unroll
-                    for (int l = 0; l < N1; ++l) v += sDm[pos * N1 + l] * u[s * NP + base + l * st];
-                    if (pos == 0) {
-                        const R ue = sT[((c * 6 + 2 * d) * 5 + s) * NF + fn];
-                        v += co.inv_wend * (-(R(0.5) * (u[s * NP + node] + ue) - u[s * NP + node]));
-                    }
-                    if (pos == N1 - 1) {
-                        const R ue = sT[((c * 6 + 2 * d + 1) * 5 + s) * NF + fn];
-                        v += co.inv_wend * ((R(0.5) * (u[s * NP + node] + ue) - u[s * NP + node]));
-                    }
-                    g[s][d] = v * inv_h;
-                }
-            }
-            R un[5];
-#pragma unroll
-            for (int s = 0; s < 5; ++s) un[s] = u[s * NP + node];
-            R F[3][4];
-            if constexpr (CURV) aux_curv_flux<R, N1>(un, g, metric, cell, node, pc.use_const_visc, cst, F);
-            else viscous_flux<R>(un, g, pc.use_const_visc, cst, F, 7, nullptr);
-            if constexpr (BND) aux_boundary_node<R, N1>(nbr, btype, Fb, cell, node, un, g, pc, pen, CURV ? metric : nullptr);
-#pragma unroll
-            for (int d = 0; d < 3; ++d)
-#pragma unroll
-                for (int k = 0; k < 4; ++k) sF[(c * 12 + d * 4 + k) * NP + node] = F[d][k];
-        }
-        __syncthreads();
-        for (int it = tid; it < CPC * NP; it += NT) {
-            const int c = it / NP, node = it % NP;
-            const int cell = cell0 + c;
-            if (cell >= nc) continue;
-            const int cx[3] = {node % N1, (node / N1) % N1, node / (N1 * N1)};
-            const R* Fc = sF + c * 12 * NP;
-            R* out = Fv + (size_t)cell * VT;
-            R div[4] = {R(0), R(0), R(0), R(0)};
-#pragma unroll
-            for (int d = 0; d < 3; ++d) {
-                const int st = (d == 0) ? 1 : (d == 1) ? N1 : N1 * N1;
-                const int pos = cx[d];
-                const int base = node - pos * st;
-#pragma unroll
-                for (int l = 0; l < N1; ++l) {
-                    const R coef = sDm[pos * N1 + l];
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) div[k] += coef * Fc[(d * 4 + k) * NP + base + l * st];
-                }
-                if (pos == 0 || pos == N1 - 1) {
-                    const int f = 2 * d + (pos == 0 ? 0 : 1);
-                    const int t1 = (d == 0) ? 1 : 0, t2 = (d == 2) ? 1 : 2;
-                    const int fn = cx[t2] * N1 + cx[t1];
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) out[4 * NP + (f * 4 + k) * NF + fn] = Fc[(d * 4 + k) * NP + node];
-                }
-            }
-#pragma unroll
-            for (int k = 0; k < 4; ++k) out[k * NP + node] = div[k];
         }
     }
 }
