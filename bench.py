@@ -126,7 +126,7 @@ def measured_fp64_mix(p: int, viscous: bool, precision: str):
         return None
     with open(path) as f:
         d = json.load(f)
-    return d.get(f"residual_kernel/{'navier_stokes' if viscous else 'euler'}/p{p}/{precision}")
+    return d.get(f"line_kernel/{'navier_stokes' if viscous else 'euler'}/p{p}/{precision}")
 
 
 class ClockSampler:
@@ -244,7 +244,7 @@ def ncu_traffic(p: int, viscous: bool, precision: str, ndofs: int):
         return None
     with open(path) as f:
         d = json.load(f)
-    e = d.get(f"residual_kernel/{'navier_stokes' if viscous else 'euler'}/p{p}/{precision}")
+    e = d.get(f"line_kernel/{'navier_stokes' if viscous else 'euler'}/p{p}/{precision}")
     if not e:
         return None
     return {"bytes_per_launch": e["bytes_per_dof"] * ndofs, "bytes_per_dof": e["bytes_per_dof"],
@@ -828,7 +828,8 @@ def main():
                          "unit": "TFLOP/s", "frac": alg_tflops / gemm_tflops,
                          "traffic": traffic["bytes_per_launch"] if traffic else None,   # DRAM bytes per launch
                          "traffic_detail": traffic,
-                         "kernel": "residual_kernel (stage: residual + mass inverse + RK update)",
+                         "kernel": ("gl_line_stage_kernel" if "_gl_" in args.workload else "line_kernel") +
+                                   " (stage: residual + mass inverse + RK update)",
                          "kernel_ms": stage_ms, "aux_kernel_ms": aux_ms,
                          "kernel_ms_source": "mean over the timed steps: CUDA events recorded by graph nodes "
                                              "around each kernel of every replayed RK step (ph_set_timing mode 2)"
