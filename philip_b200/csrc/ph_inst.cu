@@ -29,6 +29,10 @@ static cudaError_t launch_one(const StageArgs& a, cudaStream_t s) {
     return cudaGetLastError();
 }
 
+// cells per CTA of line_kernel's wide form (0: none; at N1 = 5 the narrow form is as fast on small meshes, at
+// N1 = 7 three directions exceed a CTA)
+template <int N1> constexpr int wide_cells() { return N1 == 2 ? 4 : N1 == 3 || N1 == 4 || N1 == 6 ? 1 : 0; }
+
 template <typename R, int N1, bool VISC, bool CURV>
 static cudaError_t launch_line(const StageArgs& a, cudaStream_t s) {
     constexpr int CPC = line_cells<N1>();
@@ -44,8 +48,34 @@ static cudaError_t launch_line(const StageArgs& a, cudaStream_t s) {
         configured[dev] = true;
     }
     const int cells = a.tiles ? a.ntiles * cells_per_cta<N1>() : a.nc - a.cell_begin;
+    if (cells <= 0) return a.tiles ? cudaSuccess : cudaErrorInvalidValue;
+    // The wide form (same bits) while its CTAs are one wave: a launch then takes one tile's chain of dependent
+    // operations, and a third of it. B200, FP64, us, narrow / wide: p = 3 12.3 / 8.2 at 4^3 to 8^3 cells, 14.3 /
+    // 12.8 at 10^3 (740 cells are a wave), 16.4 / 17.6 at 12^3, 28.9 / 32.9 at 16^3; p = 2 10.3 / 8.2 at 8^3,
+    // 10.3 / 12.3 at 10^3; p = 1 16.4 / 8.2 up to 12^3; p = 5 12.3 / 8.2 up to 5^3, 14.3 / 14.3 at 6^3 (148 a wave).
+    if constexpr (wide_cells<N1>() > 0) {
+        constexpr int CW = wide_cells<N1>();
+        using LW = LineLayout<R, N1, CW, CURV, true>;
+        constexpr size_t wbytes = LW::bytes;
+        auto wide = line_kernel<R, N1, CW, VISC, CURV, true>;
+        static int wave[64] = {0};
+        if (dev < 64 && !wave[dev]) {
+            cudaError_t e = cudaFuncSetAttribute(wide, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)wbytes);
+            if (e != cudaSuccess) return e;
+            int per_sm = 0, sms = 0;
+            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, wide, LW::NT, wbytes);
+            if (e != cudaSuccess) return e;
+            e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+            if (e != cudaSuccess) return e;
+            wave[dev] = per_sm * sms;
+        }
+        const int wgrid = (cells + CW - 1) / CW;
+        if (dev < 64 && wgrid <= wave[dev]) {
+            wide<<<wgrid, LW::NT, wbytes, s>>>(a, cells_per_cta<N1>());
+            return cudaGetLastError();
+        }
+    }
     const int grid = (cells + CPC - 1) / CPC;
-    if (grid <= 0) return a.tiles ? cudaSuccess : cudaErrorInvalidValue;
     kern<<<grid, L::NT, bytes, s>>>(a, cells_per_cta<N1>());
     return cudaGetLastError();
 }

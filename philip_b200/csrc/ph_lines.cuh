@@ -37,11 +37,13 @@ template <int N1> __host__ __device__ constexpr int line_npl() { return N1 % 2 =
 template <int N1> __host__ __device__ constexpr int line_lanes() { return N1 / line_npl<N1>(); }
 template <int N1> __host__ __device__ constexpr int line_spw() { return 32 / line_lanes<N1>(); }
 
-template <typename R, int N1, int CPC, bool CURV>
+template <typename R, int N1, int CPC, bool CURV, bool WIDE = false>
 struct LineLayout {
     static constexpr int NP = N1 * N1 * N1, NF = N1 * N1;
     static constexpr int NPL = line_npl<N1>(), H = line_lanes<N1>(), SPW = line_spw<N1>();
-    static constexpr int NT = (CPC * NF + SPW - 1) / SPW * 32;
+    static constexpr int LNT = (CPC * NF + SPW - 1) / SPW * 32;   // threads of one direction's lines
+    static constexpr int NT = (WIDE ? 3 : 1) * LNT;
+    static constexpr int NA = WIDE ? 15 : 5;                  // rows of volume terms (wide: each direction its own)
     static constexpr int NQ = 8 + (CURV ? 9 : 0);   // rho/2 v/2 (3) p E b |v|^2/4 (+ half the metric cofactor)
     static constexpr bool F32 = sizeof(R) == 4;
     // nodes of a cell in shared memory: x + N1 y + ZP z. A padded z pitch and lanes ordered by their place on
@@ -53,8 +55,8 @@ struct LineLayout {
     static constexpr int oB = oS + N1 * N1 + N1;              // (M+K)^-1 diag(w)
     static constexpr int oQ = (oB + N1 * N1 + 1) & ~1;
     static constexpr int oL = oQ + CPC * NQ * NS;             // [c][2][NS] logarithms of rho and b
-    static constexpr int oA = oL + CPC * 2 * NS;              // [c][5][NS] volume terms
-    static constexpr int oT = oA + CPC * 5 * NS;              // [c][face][5][NF] lifted face terms
+    static constexpr int oA = oL + CPC * 2 * NS;              // [c][NA][NS] volume terms
+    static constexpr int oT = oA + CPC * NA * NS;             // [c][face][5][NF] lifted face terms
     static constexpr int total = oT + CPC * 30 * NF;
     static constexpr size_t bytes = (size_t)total * sizeof(R);
     // CTAs per SM asked of the register allocator, from timing one stage on B200 (viscous, affine):
@@ -65,7 +67,7 @@ struct LineLayout {
     static constexpr int ASKED = F32 ? (N1 == 7 ? 2 : 8)
                                : N1 == 7 ? 1 : N1 == 2 ? 7 : N1 == 3 ? 5 : N1 == 6 ? (CURV ? 4 : 5) : CURV && N1 == 4 ? 3 : 4;
     // (the batched tile shapes are wider)
-    static constexpr int MINB = ASKED * NT > 2048 ? 2048 / NT : ASKED;
+    static constexpr int MINB = WIDE ? (NT <= 160 ? 3 : 1) : ASKED * NT > 2048 ? 2048 / NT : ASKED;
 };
 
 __device__ __forceinline__ int hi_word(double x) { return __double2hiint(x); }
@@ -262,9 +264,10 @@ template <int CPC> struct LineShared {
     int span[4];
 };
 
-template <typename R, int N1, int CPC, bool VISC, bool CURV>
+template <typename R, int N1, int CPC, bool VISC, bool CURV, bool WIDE = false>
 __device__ __forceinline__ void line_tile(const StageArgs& a, LineShared<CPC>& sh) {
-    using L = LineLayout<R, N1, CPC, CURV>;
+    using L = LineLayout<R, N1, CPC, CURV, WIDE>;
+    constexpr int NA = L::NA;
     constexpr int NP = L::NP, NF = L::NF, NT = L::NT, NQ = L::NQ, H = L::H, NPL = L::NPL, NS = L::NS, ZP = L::ZP;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     R* sm = reinterpret_cast<R*>(smem_raw);
@@ -432,16 +435,17 @@ __device__ __forceinline__ void line_tile(const StageArgs& a, LineShared<CPC>& s
     {
         const int lane = tid & 31;
         const int pos = lane / L::SPW < H ? lane / L::SPW : 0, seg = lane % L::SPW;   // place on the line, line
-        const int lineid = (tid >> 5) * L::SPW + seg;
+        const int dir = WIDE ? tid / L::LNT : 0;   // wide: the direction of this warp
+        const int lineid = ((tid - dir * L::LNT) >> 5) * L::SPW + seg;
         const bool lvalid = lane < H * L::SPW && lineid < CPC * NF;   // (idle lanes run along on line 0)
         const int lc = lvalid ? lineid / NF : 0, line = lvalid ? lineid - lc * NF : 0;
         const R* Qc = sQ + lc * NQ * NS;
         const R* Lc = sL + lc * 2 * NS;
-        R* Ac = sA + lc * 5 * NS;
+        R* Ac = sA + (lc * NA + 5 * dir) * NS;
         auto directions = [&](auto lm) {
             constexpr int LM = decltype(lm)::value;
 #pragma unroll 1
-            for (int d = 0; d < 3; ++d) {
+            for (int d = dir; d < (WIDE ? dir + 1 : 3); ++d) {
                 const int st = d == 0 ? 1 : d == 1 ? N1 : ZP;
                 const int la = line % N1, lb = line / N1;
                 const int base = d == 0 ? N1 * la + ZP * lb : d == 1 ? la + ZP * lb : la + N1 * lb;
@@ -450,14 +454,14 @@ __device__ __forceinline__ void line_tile(const StageArgs& a, LineShared<CPC>& s
                 R acc[NPL][5];
                 line_pairs<R, N1, NS, CURV, LM>(LineRows<R>{Qc, Qc + 6 * NS, Lc, Qc + (8 + d) * NS, r1, r2, r3}, base, st,
                                                 pos, seg, sS, cst, acc);
-                if (d > 0) __syncthreads();   // the previous direction's terms are in place
+                if (!WIDE && d > 0) __syncthreads();   // the previous direction's terms are in place
                 if (lvalid) {
                     const int row[5] = {0, r1, r2, r3, 4 * NS};
 #pragma unroll
                     for (int e = 0; e < NPL; ++e) {
                         R* A0 = Ac + base + (NPL * pos + e) * st;
 #pragma unroll
-                        for (int s = 0; s < 5; ++s) A0[row[s]] = d == 0 ? acc[e][s] : A0[row[s]] + acc[e][s];
+                        for (int s = 0; s < 5; ++s) A0[row[s]] = WIDE || d == 0 ? acc[e][s] : A0[row[s]] + acc[e][s];
                     }
                 }
             }
@@ -493,10 +497,10 @@ __device__ __forceinline__ void line_tile(const StageArgs& a, LineShared<CPC>& s
 #pragma unroll
             for (int k = 0; k < 4; ++k) dv[k] = __ldg(&p[k * NP]);
         }
-        R* A = sA + c * 5 * NS + node + (node / NF) * (ZP - NF);
+        R* A = sA + c * NA * NS + node + (node / NF) * (ZP - NF);
         R G[5];
 #pragma unroll
-        for (int s = 0; s < 5; ++s) G[s] = -A[s * NS];
+        for (int s = 0; s < 5; ++s) G[s] = WIDE ? -((A[s * NS] + A[(5 + s) * NS]) + A[(10 + s) * NS]) : -A[s * NS];
         if constexpr (VISC) {
 #pragma unroll
             for (int k = 0; k < 4; ++k) G[1 + k] -= dv[k];
@@ -536,7 +540,7 @@ __device__ __forceinline__ void line_tile(const StageArgs& a, LineShared<CPC>& s
     if (!inv) return;
     // FR mass inverse B (x) B (x) B, direction by direction, between the volume terms' rows and the
     // node quantities' rows (curvilinear: the weight-adjusted inverse, 1 / det J between two applications)
-    constexpr int SRC = 5 * NS, DST = NQ * NS;
+    constexpr int SRC = NA * NS, DST = NQ * NS;
     R* src = sA;
     R* dst = sQ;
     int ns = SRC, nd = DST;
@@ -606,14 +610,16 @@ __device__ __forceinline__ int line_cell(const StageArgs& a, int slot, int tc) {
     return cell < a.nc ? cell : -1;
 }
 
-template <typename R, int N1, int CPC, bool VISC, bool CURV>
-__global__ void __launch_bounds__(LineLayout<R, N1, CPC, CURV>::NT, LineLayout<R, N1, CPC, CURV>::MINB)
+// Wide form: one warp group per direction instead of one after the other, for meshes whose cells do not fill
+// the SMs with warps and whose time is one tile's chain of dependent operations.
+template <typename R, int N1, int CPC, bool VISC, bool CURV, bool WIDE = false>
+__global__ void __launch_bounds__(LineLayout<R, N1, CPC, CURV, WIDE>::NT, LineLayout<R, N1, CPC, CURV, WIDE>::MINB)
 line_kernel(const StageArgs a, int tc) {
     __shared__ LineShared<CPC> sh;
     if (threadIdx.x < CPC) sh.cell[threadIdx.x] = line_cell(a, (int)blockIdx.x * CPC + (int)threadIdx.x, tc);
     if (threadIdx.x < 4) sh.span[threadIdx.x] = (threadIdx.x & 1) ? (int)0x80000000 : 0x7fffffff;
     __syncthreads();
-    line_tile<R, N1, CPC, VISC, CURV>(a, sh);
+    line_tile<R, N1, CPC, VISC, CURV, WIDE>(a, sh);
 }
 
 // The batched form (residual_kernel_batched's tile list and instance table) over the same tile.
