@@ -118,15 +118,27 @@ def flops_per_dof_stage(p: int, viscous: bool) -> dict:
             "rule": "add/mul 1, fma 2, div/sqrt/log 1; each node pair and each face once"}
 
 
-def measured_fp64_mix(p: int, viscous: bool, precision: str):
+def stage_kernels(workload: str, boundaries=None):
+    """The stage kernels a workload runs: the periodic tiles' one, and beside it the boundary-face one where
+    a side is not periodic."""
+    gl = "_gl_" in workload
+    names = ["gl_line_stage_kernel" if gl else "line_kernel"]
+    if boundaries and any(b not in ("periodic", 0) for b in boundaries):
+        names.append("gl_stage_kernel" if gl else "residual_kernel")
+    return names
+
+
+def measured_fp64_mix(kernels, p: int, viscous: bool, precision: str):
     """Executed FP64 operations and FP64-pipe activity of the stage kernel from an ncu capture
-    (profiles/fp64_mix.json), or None."""
+    (profiles/fp64_mix.json), or None when no capture is of the one kernel that runs."""
+    if len(kernels) != 1:
+        return None
     path = os.path.join(ROOT, "profiles", "fp64_mix.json")
     if not os.path.exists(path):
         return None
     with open(path) as f:
         d = json.load(f)
-    return d.get(f"line_kernel/{'navier_stokes' if viscous else 'euler'}/p{p}/{precision}")
+    return d.get(f"{kernels[0]}/{'navier_stokes' if viscous else 'euler'}/p{p}/{precision}")
 
 
 class ClockSampler:
@@ -235,16 +247,18 @@ def gemm_peak(torch, dtype):
     return 2.0 * n ** 3 / (best * 1e-3) / 1e12
 
 
-def ncu_traffic(p: int, viscous: bool, precision: str, ndofs: int):
+def ncu_traffic(kernels, p: int, viscous: bool, precision: str, ndofs: int):
     """DRAM bytes (read + write) of one stage-kernel launch, from the ncu capture summarised
-    in profiles/dram_traffic.json (bytes per DOF of a smaller case of the same order and
-    physics, scaled by the DOFs of this workload), or None when no capture matches."""
+    in profiles/dram_traffic.json (bytes per DOF of a case of the same order and physics, scaled
+    by the DOFs of this workload), or None when no capture is of the one kernel that runs."""
+    if len(kernels) != 1:
+        return None
     path = os.path.join(ROOT, "profiles", "dram_traffic.json")
     if not os.path.exists(path):
         return None
     with open(path) as f:
         d = json.load(f)
-    e = d.get(f"line_kernel/{'navier_stokes' if viscous else 'euler'}/p{p}/{precision}")
+    e = d.get(f"{kernels[0]}/{'navier_stokes' if viscous else 'euler'}/p{p}/{precision}")
     if not e:
         return None
     return {"bytes_per_launch": e["bytes_per_dof"] * ndofs, "bytes_per_dof": e["bytes_per_dof"],
@@ -790,16 +804,17 @@ def main():
         bpd = bytes_per_dof_stage(viscous, p)
         if args.precision == "fp32":
             pass   # the state stays FP64, so the stage bytes are the same (+8 B/DOF Kahan term at the last stage)
+        kernels = stage_kernels(args.workload, args.bnd)
+        traffic = ncu_traffic(kernels, p, viscous, args.precision, dg.n_dofs)
+        # the byte and operation models are the collocated stage kernel's: no roofline figure on GL nodes
+        modelled = "_gl_" not in args.workload
         bytes_launch = bpd["stage"] * dg.n_dofs
-        achieved_gbs = bytes_launch / (stage_ms * 1e-3) / 1e9
-        traffic = ncu_traffic(p, viscous, args.precision, dg.n_dofs)
+        achieved_gbs = bytes_launch / (stage_ms * 1e-3) / 1e9 if modelled else None
         flops = flops_per_dof_stage(p, viscous)
-        alg_tflops = flops["per_dof"] * dg.n_dofs / (stage_ms * 1e-3) / 1e12
+        alg_tflops = flops["per_dof"] * dg.n_dofs / (stage_ms * 1e-3) / 1e12 if modelled else None
         fp32 = args.precision == "fp32"
         gemm_tflops = gemm_peak(torch, torch.float32 if fp32 else torch.float64)
-        mix = measured_fp64_mix(p, viscous, args.precision)
-        if "_gl_" in args.workload:   # the byte and flop models above are the collocated kernel's
-            flops = dict(flops, applies_to="collocated (GLL) stage kernel; this workload runs the GL kernels")
+        mix = measured_fp64_mix(kernels, p, viscous, args.precision)
         line = {
             "metric": "TGV DOF-updates/s/stage", "value": value, "unit": "DOF-updates/s/stage",
             "n_gpus": world, "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms_per_step,
@@ -825,21 +840,20 @@ def main():
             # the binding roof of the stage kernel is its floating-point pipe (arithmetic intensity
             # above the HBM ridge); the HBM figures are kept beside it
             "roofline": {"bound": "fp32" if fp32 else "fp64", "achieved": alg_tflops, "peak": gemm_tflops,
-                         "unit": "TFLOP/s", "frac": alg_tflops / gemm_tflops,
+                         "unit": "TFLOP/s", "frac": alg_tflops / gemm_tflops if modelled else None,
                          "traffic": traffic["bytes_per_launch"] if traffic else None,   # DRAM bytes per launch
                          "traffic_detail": traffic,
-                         "kernel": ("gl_line_stage_kernel" if "_gl_" in args.workload else "line_kernel") +
-                                   " (stage: residual + mass inverse + RK update)",
+                         "kernel": " + ".join(kernels) + " (stage: residual + mass inverse + RK update)",
                          "kernel_ms": stage_ms, "aux_kernel_ms": aux_ms,
                          "kernel_ms_source": "mean over the timed steps: CUDA events recorded by graph nodes "
                                              "around each kernel of every replayed RK step (ph_set_timing mode 2)"
                                              if not slab else "per-launch CUDA events after the timed steps",
-                         "alg_flops_per_dof": flops,
+                         "alg_flops_per_dof": flops if modelled else None,
                          "peak_source": ("measured here: cuBLAS " + ("SGEMM (TF32 off)" if fp32 else "DGEMM")
                                          + " 8192^3, best of 3; MEASURED_PEAKS.json holds no FP64/FP32 figure"),
                          "executed": mix,
                          "hbm": {"achieved": achieved_gbs, "peak": peak, "unit": "GB/s", "frac": achieved_gbs / peak,
-                                 "alg_bytes_per_dof": bpd, "peak_source": peak_src}},
+                                 "alg_bytes_per_dof": bpd, "peak_source": peak_src} if modelled else None},
             "clocks": clk.summary(),
         }
         if world == 1 and not args.no_served_sample and not slab:
