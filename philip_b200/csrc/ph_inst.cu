@@ -50,9 +50,12 @@ static cudaError_t launch_line(const StageArgs& a, cudaStream_t s) {
     const int cells = a.tiles ? a.ntiles * cells_per_cta<N1>() : a.nc - a.cell_begin;
     if (cells <= 0) return a.tiles ? cudaSuccess : cudaErrorInvalidValue;
     // The wide form (same bits) while its CTAs are one wave: a launch then takes one tile's chain of dependent
-    // operations, and a third of it. B200, FP64, us, narrow / wide: p = 3 12.3 / 8.2 at 4^3 to 8^3 cells, 14.3 /
-    // 12.8 at 10^3 (740 cells are a wave), 16.4 / 17.6 at 12^3, 28.9 / 32.9 at 16^3; p = 2 10.3 / 8.2 at 8^3,
-    // 10.3 / 12.3 at 10^3; p = 1 16.4 / 8.2 up to 12^3; p = 5 12.3 / 8.2 up to 5^3, 14.3 / 14.3 at 6^3 (148 a wave).
+    // operations, and a third of it. At p = 1, where the narrow form's CTAs hold 16 cells in two warps, while they
+    // are two waves. B200, us per RK4 step (four launches, Navier-Stokes eight), narrow / wide, FP64 Euler:
+    //   p = 3  43 / 23 at 4^3 cells, 49 / 33 at 9^3, 57 / 68 at 12^3    p = 2  35 / 29 at 9^3, 37 / 43 at 10^3
+    //   p = 5  41 / 27 at 5^3, 47 / 49 at 6^3, 57 / 69 at 7^3           p = 1  64 / 45 at 16^3, 68 / 51 at 19^3, 78 / 84 at 23^3
+    // Navier-Stokes p = 3 74 / 55 at 9^3, 96 / 103 at 12^3; curved p = 3 53 / 35 at 9^3, 66 / 74 at 12^3; precision form
+    // (fewer registers, so more CTAs a wave) p = 3 47 / 33 at 11^3, 59 / 68 at 14^3, p = 1 60 / 49 at 21^3, 64 / 66 at 23^3.
     if constexpr (wide_cells<N1>() > 0) {
         constexpr int CW = wide_cells<N1>();
         using LW = LineLayout<R, N1, CW, CURV, true>;
@@ -69,8 +72,9 @@ static cudaError_t launch_line(const StageArgs& a, cudaStream_t s) {
             if (e != cudaSuccess) return e;
             wave[dev] = per_sm * sms;
         }
+        constexpr int WAVES = N1 == 2 ? 2 : 1;
         const int wgrid = (cells + CW - 1) / CW;
-        if (dev < 64 && wgrid <= wave[dev]) {
+        if (dev < 64 && wgrid <= WAVES * wave[dev]) {
             wide<<<wgrid, LW::NT, wbytes, s>>>(a, cells_per_cta<N1>());
             return cudaGetLastError();
         }
