@@ -66,8 +66,23 @@ struct LineLayout {
     // cells, 4: 0.113). Curvilinear cells' rows leave room for fewer CTAs at N1 = 4 and 6.
     static constexpr int ASKED = F32 ? (N1 == 7 ? 2 : 8)
                                : N1 == 7 ? 1 : N1 == 2 ? 7 : N1 == 3 ? 5 : N1 == 6 ? (CURV ? 4 : 5) : CURV && N1 == 4 ? 3 : 4;
-    // (the batched tile shapes are wider)
-    static constexpr int MINB = WIDE ? (NT <= 160 ? 3 : 1) : ASKED * NT > 2048 ? 2048 / NT : ASKED;
+    static constexpr int MINB = WIDE ? (NT <= 160 ? 3 : 1) : ASKED;
+    // The batched kernel's own: its arguments come from shared memory, not from the parameter bank, which takes
+    // registers, and its tiles may be wider. Timed on B200, one stage of 24^3 cells (16^3 from N1 = 5), us,
+    // affine / curved, the single kernel's request -> this one, where they differ:
+    //   precision form  N1 = 3, 8 cells 56 / 83 -> 41 / 60   N1 = 4, 2 cells 82 / 138 -> 71 / 111, 4 cells 74 / 115 -> 72 / 115
+    //                   N1 = 5, 2 cells 71 / 99 -> 58 / 82   N1 = 6 80 / 133 -> 78 / 122   N1 = 7 157 / 227 -> 154 / 202
+    //   FP64            N1 = 2 25 -> 23 (affine)             N1 = 3, 4 cells 60 / 94 -> 58 / 89, 8 cells 80 / 122 -> 60 / 93
+    //                   N1 = 4, 2 cells 144 / 258 -> 105 / 192   N1 = 5, 1 cell 76 / 121 -> 74 / 119, 2 cells 85 / 136 -> 80 / 121
+    //                   N1 = 6 119 -> 115 (affine)           N1 = 7 303 / 486 -> 227 / 337
+    // Some of these spill (FP64 up to 230 bytes of local memory a thread at N1 = 3, 5 and 7): the requests that do
+    // not leave too few warps (N1 = 5, 1 cell, FP64: none at 2 CTAs per SM, 109 us; 120 bytes at 5, 74 us).
+    static constexpr int BATCHED =
+        N1 == 2 ? (F32 ? 8 : CURV ? 5 : 6)
+        : N1 == 3 ? (CPC == 4 ? (F32 ? (CURV ? 8 : 7) : 6) : F32 ? 4 : 3)
+        : N1 == 4 ? (CPC == 2 ? (F32 ? (CURV ? 12 : 14) : CURV ? 6 : 8) : F32 ? (CURV ? 6 : 7) : CURV ? 3 : 4)
+        : N1 == 5 ? (CPC == 1 ? (F32 ? 8 : 5) : F32 ? 4 : 3)
+        : N1 == 6 ? (F32 ? (CURV ? 7 : 6) : 4) : F32 ? 3 : 2;
 };
 
 __device__ __forceinline__ int hi_word(double x) { return __double2hiint(x); }
@@ -624,7 +639,7 @@ line_kernel(const StageArgs a, int tc) {
 
 // The batched form (residual_kernel_batched's tile list and instance table) over the same tile.
 template <typename R, int N1, int CPC, bool CURV>
-__global__ void __launch_bounds__(LineLayout<R, N1, CPC, CURV>::NT, LineLayout<R, N1, CPC, CURV>::MINB)
+__global__ void __launch_bounds__(LineLayout<R, N1, CPC, CURV>::NT, LineLayout<R, N1, CPC, CURV>::BATCHED)
 line_kernel_batched(const StageArgs* __restrict__ inst, const BatchTile* __restrict__ tiles, int ntiles) {
     __shared__ __align__(16) StageArgs sa;
     __shared__ LineShared<CPC> sh;
