@@ -1574,7 +1574,7 @@ gl_cons_stage_kernel(const StageArgs a, const GlArgs g, const __grid_constant__ 
 // while the node quantities are formed. The temporaries of the final passes reuse the space of the
 // quantities (48 KB at NQ = 6: four CTAs per SM). At 12^3 cells of p = 5 it takes 86 us
 // (FP64 pipe 37 % busy, the rest latency), 97 us while the faces were lifted one after the other after
-// the last interpolation. A three-stage step of 24^3 such cells: 11.9 ms with the node form, 7.7 with
+// the last interpolation. An RK4 step of 24^3 such cells: 11.9 ms with the node form, 7.7 with
 // this kernel and the states projected once, 4.9 with the line form of the other two kernels.
 template <int ND, int NQ>
 struct GlLineLayout {

@@ -357,8 +357,10 @@ __global__ void integrals_kernel(const double* __restrict__ U, const double* __r
 // centre, so the column is held as even and odd halves and two mirrored points share their sums:
 // 4 operations per field and point at N1 = 6 instead of 6. The factors 1 / h and the cell's volume
 // are taken out of the sums; the wave speed is compared squared (one root per point).
-// Bound by FP64 operations of few warps with much independent work. A step of 16^3 cells of p = 5 with its
-// integrals takes 1.02 ms where the field-by-field contraction at every point took 1.30.
+// Bound by FP64 operations of few warps with much independent work. One call at 16^3 cells on B200, its four numbers'
+// way to the host included, field-by-field contraction at every point -> this kernel: p = 1 0.163 -> 0.090 ms, p = 2
+// 0.222 -> 0.125, p = 3 0.345 -> 0.208, p = 4 0.579 -> 0.272, p = 5 0.641 -> 0.350, p = 6 1.35 -> 1.06 (its column of 77
+// values does not fit the 168 registers that ten warps leave: 2.2 KB a thread are spilled).
 template <int N1> struct IntegralsAffine {
     static constexpr int NE = N1 + 10, NP = N1 * N1 * N1, NT2 = N1 * N1 * NE;
     static constexpr int NT = (NE * NE + 31) / 32 * 32;

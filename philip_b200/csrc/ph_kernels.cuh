@@ -1135,10 +1135,10 @@ residual_kernel_batched(const StageArgs* __restrict__ inst, const BatchTile* __r
 // An FR auxiliary correction (K_aux != 0) multiplies the gradient by Baux(x)Baux(x)Baux before
 // the flux.
 
-// CTAs per SM of the periodic FP64 auxiliary kernel at p = 5 (224 threads). Timed on B200 at
-// 24^3 cells inside the RK4 steps: 3 (76 registers) 0.163 ms, 4 (70 registers) 0.147 ms, 5 (56
-// registers, 32 bytes spilled) 0.155 ms. Asked for explicitly: launch bounds naming 1 CTA per SM
-// gave 76 registers, and the allocator's choice without a count sits at 70.
+// CTAs per SM of the periodic FP64 auxiliary kernel at p = 5 (224 threads): 66 registers, 0.140 ms at 24^3
+// cells. Chosen on B200 before the lines along x moved in pairs: 3 (76 registers) 0.163 ms, 4 (70
+// registers) 0.147 ms, 5 (56 registers, 32 bytes spilled) 0.155 ms. Asked for explicitly: launch
+// bounds naming 1 CTA per SM gave 76 registers.
 #ifndef PH_AUX_P5_MINB
 #define PH_AUX_P5_MINB 4
 #endif

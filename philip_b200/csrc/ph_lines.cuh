@@ -6,16 +6,16 @@
 // of the line is evaluated once and every lane evaluates equally many (N1 = 6: five pairs on each of
 // three lanes, its own pair and the four with the next lane's nodes; a pair's flux goes to the
 // next lane by shuffles). The three directions run one after the other through one copy of the code.
-// Neighbour face values are gathered into registers while the node quantities are formed, and face
-// fluxes go through shared memory once, as lifted terms.
+// A neighbour's face values are read where the face fluxes are evaluated, and those go through shared memory
+// once, as lifted terms.
 //
 // Why this split, against the node-per-lane form (residual_kernel): no pair of an even line is
 // evaluated twice (15 instead of 18 per line at N1 = 6), the logarithms of the means are taken only in
 // tiles whose gradients need them, halved node quantities save six operations per pair, the
 // neighbour traces take no shared memory, and the rolled direction loop keeps the code in the
-// instruction caches. The operations and their order per node are the same, so both kernels give the
-// same bits. What bounds it: FP64 operations with dependent latencies (FP64 pipe 46 %, issue 53 %, 19
-// of 64 warps at 24^3 cells, p = 5); in the precision form issue slots (69 %).
+// instruction caches. The operations and their order per node are the same, so in FP64 both kernels give
+// the same bits. What bounds it: FP64 operations with dependent latencies (FP64 pipe 44 %, issue 53 %, 19
+// of 64 warps at 24^3 cells, p = 5); in the precision form issue slots (70 %).
 // One stage, viscous, B200, node-per-lane form -> this kernel (FP64 / precision form, ms):
 //   24^3 cells p = 5  0.488 -> 0.320 / 0.269 -> 0.215    32^3 p = 3  0.385 -> 0.224 / 0.215 -> 0.142
 //   24^3 p = 4        0.305 -> 0.217 / 0.176 -> 0.132    30^3 p = 2  0.183 -> 0.105 / 0.111 -> 0.070
@@ -70,7 +70,7 @@ struct LineLayout {
     // The batched kernel's own: its arguments come from shared memory, not from the parameter bank, which takes
     // registers, and its tiles may be wider. Timed on B200, one stage of 24^3 cells (16^3 from N1 = 5), us,
     // affine / curved, the single kernel's request -> this one, where they differ:
-    //   precision form  N1 = 3, 8 cells 56 / 83 -> 41 / 60   N1 = 4, 2 cells 82 / 138 -> 71 / 111, 4 cells 74 / 115 -> 72 / 115
+    //   precision form  N1 = 3, 8 cells 56 / 83 -> 41 / 60   N1 = 4, 2 cells 82 / 138 -> 71 / 111, 4 cells 74 / 122 -> 72 / 115
     //                   N1 = 5, 2 cells 71 / 99 -> 58 / 82   N1 = 6 80 / 133 -> 78 / 122   N1 = 7 157 / 227 -> 154 / 202
     //   FP64            N1 = 2 25 -> 23 (affine)             N1 = 3, 4 cells 60 / 94 -> 58 / 89, 8 cells 80 / 122 -> 60 / 93
     //                   N1 = 4, 2 cells 144 / 258 -> 105 / 192   N1 = 5, 1 cell 76 / 121 -> 74 / 119, 2 cells 85 / 136 -> 80 / 121
